@@ -143,6 +143,34 @@ LRT_HD float lrt_exp_in_range(float x) {
 #endif
 }
 
+#if defined(__CUDACC__)
+// w lrt_exp_in_range(-power / 2) for two powers at once, in packed single
+// precision, with the bits of the scalar forms (w a positive normal number,
+// the product in range). Three things are left out that only scale by powers
+// of two, which moves no rounding: the argument's factor -1/2 (the reduced
+// argument here is -2 r, so the coefficient of r^k carries (-1/2)^k), and the
+// factor 2^n, added to w's exponent instead of multiplied in twice.
+__device__ __forceinline__ float2 lrt_scaled_exp_half2(float w, float2 power) {
+    auto both = [](float v) { return make_float2(v, v); };
+    constexpr float kMagic = 12582912.0f;   // as in lrt_exp_in_range; its bits << 23 are 0
+    const float2 t = __fadd2_rn(__fmul2_rn(power, both(-0.5f * 1.44269504088896340736f)), both(kMagic));
+    const float2 n = __fadd2_rn(t, both(-kMagic));
+    float2 r = __ffma2_rn(n, both(2.0f * 0.693147182464599609375f), power);   // -2 r
+    r = __ffma2_rn(n, both(-2.0f * 1.904654299957768e-09f), r);
+    float2 p = both(1.984126984126984e-4f / -128.0f);
+    p = __ffma2_rn(p, r, both(1.388888888888889e-3f / 64.0f));
+    p = __ffma2_rn(p, r, both(8.333333333333333e-3f / -32.0f));
+    p = __ffma2_rn(p, r, both(4.166666666666666e-2f / 16.0f));
+    p = __ffma2_rn(p, r, both(1.666666666666667e-1f / -8.0f));
+    p = __ffma2_rn(p, r, both(0.5f / 4.0f));
+    p = __ffma2_rn(p, r, both(1.0f / -2.0f));
+    p = __ffma2_rn(p, r, both(1.0f));
+    const uint32_t bits = __float_as_uint(w);
+    return __fmul2_rn(p, make_float2(__uint_as_float(bits + (__float_as_uint(t.x) << 23)),
+                                     __uint_as_float(bits + (__float_as_uint(t.y) << 23))));
+}
+#endif
+
 LRT_HD float lrt_log(float x) {
     if (x != x) return x;
     if (x < 0.0f) return NAN;
