@@ -183,7 +183,9 @@ __device__ __forceinline__ float2 upper2(float4 v) { return make_float2(v.z, v.w
 // index where it reaches the layer's depth), not from depth order.
 // Returns true when a bounded wait gave up (kErrTimeout is set): the
 // barrier's phase is then unknown, so a persistent caller must stop.
-template <bool kTrain, bool kComposite = false>
+// kWords: the pairs are 64-bit words with the slot (or emit index) in their
+// low field; else every tile's slots alone (rows.cu).
+template <bool kTrain, bool kWords, bool kComposite = false>
 __device__ __forceinline__ bool blend_tile(const BlendParams& bp, uint32_t tile, uint32_t tx, uint32_t ty,
                                            const uint2* __restrict__ ranges,
                                            const unsigned long long* __restrict__ pairs,
@@ -243,6 +245,7 @@ __device__ __forceinline__ bool blend_tile(const BlendParams& bp, uint32_t tile,
     // The record slot of the pair at `at` + this thread's index.
     auto slot_at = [&](uint32_t at) -> uint32_t {
         if (at >= end || tid >= end - at) return 0u;
+        if constexpr (!kWords) return reinterpret_cast<const uint32_t*>(pairs)[at + tid];
         uint32_t slot = static_cast<uint32_t>(pairs[at + tid] & slotMask);
         if constexpr (kTrain) {
             if (emitSlot != nullptr) slot = emitSlot[slot];   // the low field is the emit index
@@ -504,7 +507,7 @@ __device__ __forceinline__ void blend_init(BlendShared& sh) {
     __syncthreads();
 }
 
-template <bool kTrain, bool kChained>
+template <bool kTrain, bool kWords, bool kChained>
 __global__ void __launch_bounds__(kBlendThreads / kBlendPix)
 blend_kernel(BlendParams bp, const uint2* __restrict__ ranges, const unsigned long long* __restrict__ pairs,
              const uint32_t* __restrict__ emitSlot,
@@ -516,12 +519,13 @@ blend_kernel(BlendParams bp, const uint2* __restrict__ ranges, const unsigned lo
     blend_init(sh);
     uint32_t phase = 0;
     const uint32_t tile = order != nullptr ? order[blockIdx.x] : blockIdx.x;
-    blend_tile<kTrain>(bp, tile, tile % bp.tilesX, tile / bp.tilesX, ranges, pairs, emitSlot, proj, colourOut, depthOut,
+    blend_tile<kTrain, kWords>(bp, tile, tile % bp.tilesX, tile / bp.tilesX, ranges, pairs, emitSlot, proj, colourOut, depthOut,
                        pixState, pixLast, err, sh, phase);
 }
 
 // splatBlendComposite (splat_blend.slang:116-120): discs and an optional
 // under layer (colour may be null).
+template <bool kWords>
 __global__ void __launch_bounds__(kBlendThreads / kBlendPix)
 blend_composite_kernel(BlendParams bp, const uint2* __restrict__ ranges, const unsigned long long* __restrict__ pairs,
                        const ProjRecord* __restrict__ proj, float4* __restrict__ colourOut,
@@ -532,7 +536,7 @@ blend_composite_kernel(BlendParams bp, const uint2* __restrict__ ranges, const u
     blend_init(sh);
     uint32_t phase = 0;
     const uint32_t tile = blockIdx.x;
-    blend_tile<false, true>(bp, tile, tile % bp.tilesX, tile / bp.tilesX, ranges, pairs, nullptr, proj, colourOut,
+    blend_tile<false, kWords, true>(bp, tile, tile % bp.tilesX, tile / bp.tilesX, ranges, pairs, nullptr, proj, colourOut,
                             depthOut, nullptr, nullptr, err, sh, phase, underColour, underDepth, &comp);
 }
 
@@ -567,7 +571,7 @@ blend_batch_kernel(BlendParams bp, const ViewParams* __restrict__ views, uint32_
         vbp.height = v.height;
         vbp.tilesX = v.tilesX;
         const uint32_t local = item - v.tileBase;
-        const bool gaveUp = blend_tile<kTrain>(
+        const bool gaveUp = blend_tile<kTrain, true>(
             vbp, item, local % v.tilesX, local / v.tilesX, ranges, pairs, nullptr, proj + v.recordBase, v.colour,
             v.depth, kTrain ? v.pixState : nullptr, kTrain ? v.pixLast : nullptr, err, sh, phase);
         // After a wait gave up the barrier's phase is unknown: take no more
@@ -750,7 +754,10 @@ cudaError_t launch_blend(const BlendParams& bp, const uint2* ranges, const uint6
                          float4* colour, float* depth, uint32_t* err, cudaStream_t stream, const uint32_t* order) {
     const uint32_t tiles = bp.tilesX * bp.tilesY;
     if (tiles == 0) return cudaSuccess;
-    return launch_chained(blend_kernel<false, true>, blend_kernel<false, false>, dim3(tiles), dim3(kBlendThreads / kBlendPix), 0, stream, bp, ranges,
+    const bool words = bp.pairShift != 0;
+    return launch_chained(words ? blend_kernel<false, true, true> : blend_kernel<false, false, true>,
+                          words ? blend_kernel<false, true, false> : blend_kernel<false, false, false>, dim3(tiles),
+                          dim3(kBlendThreads / kBlendPix), 0, stream, bp, ranges,
                           reinterpret_cast<const unsigned long long*>(pairs), static_cast<const uint32_t*>(nullptr), proj,
                           colour, depth, static_cast<float4*>(nullptr), static_cast<uint32_t*>(nullptr), err, order);
 }
@@ -760,7 +767,8 @@ cudaError_t launch_blend_composite(const BlendParams& bp, const uint2* ranges, c
                                   const float* underDepth, uint32_t* err, cudaStream_t stream) {
     const uint32_t tiles = bp.tilesX * bp.tilesY;
     if (tiles == 0) return cudaSuccess;
-    blend_composite_kernel<<<tiles, kBlendThreads / kBlendPix, 0, stream>>>(
+    const auto kernel = bp.pairShift != 0 ? blend_composite_kernel<true> : blend_composite_kernel<false>;
+    kernel<<<tiles, kBlendThreads / kBlendPix, 0, stream>>>(
         bp, ranges, reinterpret_cast<const unsigned long long*>(pairs), proj, colour, depth, underColour, underDepth,
         err);
     return cudaGetLastError();
@@ -793,7 +801,10 @@ cudaError_t launch_blend_train(const BlendParams& bp, const uint2* ranges, const
                                const uint32_t* order) {
     const uint32_t tiles = bp.tilesX * bp.tilesY;
     if (tiles == 0) return cudaSuccess;
-    return launch_chained(blend_kernel<true, true>, blend_kernel<true, false>, dim3(tiles), dim3(kBlendThreads / kBlendPix), 0, stream, bp, ranges,
+    const bool words = bp.pairShift != 0;
+    return launch_chained(words ? blend_kernel<true, true, true> : blend_kernel<true, false, true>,
+                          words ? blend_kernel<true, true, false> : blend_kernel<true, false, false>, dim3(tiles),
+                          dim3(kBlendThreads / kBlendPix), 0, stream, bp, ranges,
                           reinterpret_cast<const unsigned long long*>(pairs), emitSlot, proj, colour, depth, pixState,
                           pixLast, err, order);
 }

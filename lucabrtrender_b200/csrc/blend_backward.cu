@@ -124,8 +124,10 @@ __device__ __forceinline__ void blend_backward_tile(const BlendParams& bp, uint3
     const uint32_t py0 = ty * kTile + (cell >> 2) * 4u;
     const uint2 range = ranges[item];
     const uint32_t start = range.x;
-    const unsigned long long slotMask = (1ull << bp.slotBits) - 1ull;
-    auto lowWord = [&](uint32_t k) { return static_cast<uint32_t>(__ldg(pairs + k) & slotMask); };   // the low field
+    const uint32_t slotMask = static_cast<uint32_t>((1ull << bp.slotBits) - 1ull);
+    auto lowWord = [&](uint32_t k) {   // a pair word's low field, or the slot alone
+        return __ldg(reinterpret_cast<const uint32_t*>(pairs) + (static_cast<size_t>(k) << bp.pairShift)) & slotMask;
+    };
     const float pxf = static_cast<float>(px) + 0.5f;
     const float tileX = static_cast<float>(tx * kTile), tileY = static_cast<float>(ty * kTile);
 

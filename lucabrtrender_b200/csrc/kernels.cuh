@@ -55,12 +55,14 @@ cudaError_t launch_project_only(const FrameParams& f, const float4* positions, c
                                 const float* filter3d, ProjRecord* proj, uint4* rects, uint32_t* touched,
                                 uint32_t* keys, uint32_t* counters, uint32_t* ticket, uint64_t* aux,
                                 uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream);
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream);
 cudaError_t launch_project_points_only(const FrameParams& f, const float4* positions, const uint32_t* colours,
                                        const lrt_point_style& style, ProjRecord* proj, uint4* rects, uint32_t* touched,
                                        uint32_t* keys, uint32_t* counters, uint32_t* ticket, uint64_t* aux,
                                        uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream);
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream);
+// runCounts, bands (null: not wanted): per slot its touched tiles and its runs
+// of them; added to bands[0 .. 255], the runs in each tile row (rows.cu).
 // rowTable (rowCap entries; counters[3] counts the entries asked for): each
 // large splat's rows (first column, count), kept by the projection for the
 // pair writes; null: none kept.
@@ -81,7 +83,38 @@ cudaError_t launch_project_only_train(const FrameParams& f, const float* means, 
                                       const float* quats, const float* logits, const uint16_t* sh, ProjRecord* proj,
                                       uint4* rects, uint32_t* touched, uint32_t* keys, uint32_t* counters,
                                       uint32_t* ticket, uint64_t* aux, uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream);
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream);
+
+// The pairs of a single frame of at most kMaxBands x kMaxBands tiles, from the
+// depth-sorted slot words (rows.cu): every tile's slots in depth order.
+struct RowFrame {
+    const uint64_t* sortedWords;   // depthKey << 32 | slot, sorted
+    uint32_t slots, width, height, tilesX, tilesY;
+    const ProjRecord* proj;
+    const uint4* rects;
+    const uint64_t* aux;           // per slot its tile mask, or a large splat's row table place
+    const uint2* rowTable;
+    const uint2* runCounts;        // per slot (touched, runs)
+    const uint32_t* bands;         // runs per tile row
+    uint32_t* counters;            // [1] pairs, [2] error bits, [4] runs
+    uint32_t* pairOffsets;         // out, training frames: each slot's first emit index (else null)
+    uint64_t* runs;                // runCap sorted runs
+    uint32_t* runEmit;             // training frames: their first emit index (else null)
+    uint32_t runCap, pairCap;
+    uint32_t* pairSlots;           // out: every tile's slots
+    uint32_t* pairEmit;            // out, training frames: the pairs' emit indices (else null)
+    uint2* ranges;                 // out (zeroed): every tile's pairs
+    void* zeroed;                  // row_zeroed_bytes(slots), zeroed
+    void* scratch;                 // row_scratch_bytes(slots, runCap, tilesX)
+};
+constexpr uint32_t kMaxBands = 256;
+size_t row_zeroed_bytes(uint32_t slots);
+size_t row_scratch_bytes(uint32_t slots, uint32_t runCap, uint32_t tilesX);
+cudaError_t launch_row_runs(const RowFrame& f, cudaStream_t stream);    // the runs, sorted by tile row
+cudaError_t launch_row_pairs(const RowFrame& f, cudaStream_t stream);   // every tile's pairs and range
+// A frame's `pairs` pairs as the debug view shows them: tile << 32 | low[k].
+cudaError_t launch_pair_words(const uint2* ranges, const uint32_t* low, uint32_t tiles, uint32_t pairs,
+                              uint64_t* words, cudaStream_t stream);
 
 size_t scan_scratch_bytes(uint32_t n);
 cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t* total, uint32_t n, void* scratch,

@@ -37,14 +37,11 @@
 // tested exactly. Pairs of masked splats are written by their warp, lanes on
 // consecutive pairs, each pair's tile from the mask bit of its rank.
 #include "kernels.cuh"
+#include "project_common.cuh"
 #include "raster_common.cuh"
-
-#include <cuda/atomic>
 
 namespace lrt {
 namespace {
-
-constexpr uint32_t kProjectThreads = 256;
 
 struct Fate {
     bool removed, graded;
@@ -288,289 +285,6 @@ struct TrainOutputs {
     uint32_t* emitSlot;
 };
 
-// Splats of up to kWarpArea tiles have their tiles tested by their warp (32
-// (splat, tile) pairs a step) and keep a 128-bit tile mask; larger ones are
-// counted and written a tile row at a time.
-constexpr uint32_t kWarpArea = 128;
-constexpr uint32_t kMaskArea = kWarpArea;
-static_assert(kMaskArea <= 128, "a tile mask has 128 bits");
-
-// ---- Splats of more than kWarpArea tiles, one tile row at a time ----
-//
-// The tiles of a row that the exact test (tile_touched) accepts are those
-// whose box of pixel centres meets the ellipse {power <= cutoff}; within the
-// row's band of pixel centres, the ellipse spans one x interval [XL, XR]. In
-// double precision that interval gives, with a margin m covering every
-// rounding of the float test (its inputs' rounding and the power's, which
-// grows with the conic's condition number), the columns that are certainly
-// touched and the few around them that must be tested exactly. A row is then
-// counted in O(1) plus a handful of exact tests, and its pairs are the
-// certain run with the exact hits either side of it: the counts and pairs
-// are the per-tile test's own, at a cost that follows the pairs, not the
-// rectangle's area. Rows near the top or bottom of the ellipse, and
-// ill-conditioned conics, are tested tile by tile.
-struct Footprint {
-    float cx, cy, a, b, c, cut;
-    uint32_t x0, x1;      // the rectangle's columns
-    uint32_t y0;          // its first row
-    uint32_t tid;         // the splat's thread in the block
-    uint32_t table;       // the splat's first row in the row table, or kNoTable
-};
-constexpr uint32_t kNoTable = 0xFFFFFFFFu;
-
-struct RowPlan {
-    int32_t lo, hi;           // candidate columns, inside the rectangle (none when lo > hi)
-    int32_t sureLo, sureHi;   // certainly touched columns, inside [lo, hi] (none when sureLo > sureHi)
-};
-
-// The x range of tile column t's pixel centres, relative to the centre, as
-// tile_touched forms it (the same float values, here exact in double).
-__device__ __forceinline__ double col_lo(int32_t t, float cx) {
-    return static_cast<double>(static_cast<float>(t * static_cast<int32_t>(kTile)) + 0.5f) - static_cast<double>(cx);
-}
-__device__ __forceinline__ double col_hi(int32_t t, uint32_t width, float cx) {
-    const int32_t last = min((t + 1) * static_cast<int32_t>(kTile), static_cast<int32_t>(width)) - 1;
-    return static_cast<double>(static_cast<float>(last) + 0.5f) - static_cast<double>(cx);
-}
-
-__device__ __forceinline__ RowPlan row_plan(const Footprint& fp, uint32_t ty, uint32_t width, uint32_t height) {
-    RowPlan p{static_cast<int32_t>(fp.x0), static_cast<int32_t>(fp.x1), 1, 0};   // default: every column exact
-    const double a = fp.a, b = fp.b, c = fp.c, k = fp.cut;
-    const double det = a * c - b * b;
-    if (!(a > 0.0) || !(c > 0.0) || !(k > 0.0) || !(det > 1e-6 * a * c)) return p;
-    const double hx = sqrt(k * c / det), hy = sqrt(k * a / det);
-    // Margin: the float test's power carries a relative error of a few
-    // roundings (4 x 2^-24) times the condition number kappa, which moves
-    // the boundary by at most that times half the long axis; its box
-    // coordinates carry one rounding of magnitudes up to |centre| + extent.
-    // Both with a factor of 8 to spare, plus a quarter pixel.
-    const double lmin = 0.5 * (a + c) - sqrt(0.25 * (a - c) * (a - c) + b * b);
-    if (!(lmin > 0.0)) return p;
-    const double kappa = (fabs(a) + 2.0 * fabs(b) + fabs(c)) / lmin;
-    const double reach = fabs(static_cast<double>(fp.cx)) + fabs(static_cast<double>(fp.cy)) + hx + hy + 64.0;
-    const double m = 0.25 + 1.0e-6 * kappa * (hx + hy) + 5.0e-7 * reach;
-    if (!(m < 24.0)) return p;
-    const int32_t ity = static_cast<int32_t>(ty);
-    const double ylo = static_cast<double>(static_cast<float>(ity * static_cast<int32_t>(kTile)) + 0.5f) -
-                       static_cast<double>(fp.cy);
-    const int32_t lastRow = min((ity + 1) * static_cast<int32_t>(kTile), static_cast<int32_t>(height)) - 1;
-    const double yhi = static_cast<double>(static_cast<float>(lastRow) + 0.5f) - static_cast<double>(fp.cy);
-    if (yhi < -hy - m || ylo > hy + m) {   // the band misses the ellipse by more than the margin
-        p.lo = 1;
-        p.hi = 0;
-        return p;
-    }
-    // Near the ellipse's top or bottom the band's x extent is ill-conditioned
-    // (it grows as the square root of the band's overlap): there the
-    // candidates are the x extent of the band widened by m on both sides,
-    // each tested exactly, and none is certain.
-    const bool tangent = yhi < -hy + m || ylo > hy - m;
-    const double bandLo = tangent ? fmax(ylo - m, -hy) : ylo;
-    const double bandHi = tangent ? fmin(yhi + m, hy) : yhi;
-    // The ellipse's x extent within the band: its leftmost and rightmost
-    // points (x = -+hx, y = -b x / c) clamped into the band.
-    const double yl = fmin(fmax(b * hx / c, bandLo), bandHi);
-    const double yr = fmin(fmax(-b * hx / c, bandLo), bandHi);
-    const double xl = (-b * yl - sqrt(fmax(k * a - det * yl * yl, 0.0))) / a;
-    const double xr = (-b * yr + sqrt(fmax(k * a - det * yr * yr, 0.0))) / a;
-    // First column whose hi >= v, and last whose lo <= v, within the
-    // rectangle (the estimate is exact but for the clipped last column; the
-    // adjustment steps are bounded and, if they do not settle, every column
-    // is tested exactly).
-    const int32_t x0 = static_cast<int32_t>(fp.x0), x1 = static_cast<int32_t>(fp.x1);
-    bool ok = true;
-    auto firstHiAtLeast = [&](double v) -> int32_t {
-        const double e = ceil((v + static_cast<double>(fp.cx) - 15.5) / 16.0);
-        int32_t t = static_cast<int32_t>(fmin(fmax(e, static_cast<double>(x0)), static_cast<double>(x1 + 1)));
-        for (int it = 0; it < 3 && t > x0 && col_hi(t - 1, width, fp.cx) >= v; ++it) --t;
-        for (int it = 0; it < 3 && t <= x1 && col_hi(t, width, fp.cx) < v; ++it) ++t;
-        if ((t > x0 && col_hi(t - 1, width, fp.cx) >= v) || (t <= x1 && col_hi(t, width, fp.cx) < v)) ok = false;
-        return t;
-    };
-    auto lastLoAtMost = [&](double v) -> int32_t {
-        const double e = floor((v + static_cast<double>(fp.cx) - 0.5) / 16.0);
-        int32_t t = static_cast<int32_t>(fmin(fmax(e, static_cast<double>(x0 - 1)), static_cast<double>(x1)));
-        for (int it = 0; it < 3 && t < x1 && col_lo(t + 1, fp.cx) <= v; ++it) ++t;
-        for (int it = 0; it < 3 && t >= x0 && col_lo(t, fp.cx) > v; ++it) --t;
-        if ((t < x1 && col_lo(t + 1, fp.cx) <= v) || (t >= x0 && col_lo(t, fp.cx) > v)) ok = false;
-        return t;
-    };
-    const int32_t lo = firstHiAtLeast(xl - m), hi = lastLoAtMost(xr + m);
-    const int32_t sureLo = tangent ? 1 : firstHiAtLeast(xl + m), sureHi = tangent ? 0 : lastLoAtMost(xr - m);
-    if (!ok) return p;
-    p.lo = lo;
-    p.hi = hi;
-    p.sureLo = tangent ? 1 : max(sureLo, lo);
-    p.sureHi = tangent ? 0 : min(sureHi, hi);
-    return p;
-}
-
-// A row's touched tiles in column order: `visit(t)` for each exact hit and
-// `run(t0, t1)` for the certain run [t0, t1].
-template <class Hit, class Run>
-__device__ __forceinline__ void row_walk(const Footprint& fp, uint32_t ty, uint32_t width, uint32_t height,
-                                         Hit&& visit, Run&& run) {
-    const RowPlan p = row_plan(fp, ty, width, height);
-    const bool sure = p.sureLo <= p.sureHi;
-    const int32_t leftEnd = sure ? p.sureLo - 1 : p.hi;
-    for (int32_t t = p.lo; t <= leftEnd; ++t)
-        if (tile_touched(width, height, fp.cx, fp.cy, fp.a, fp.b, fp.c, fp.cut, static_cast<uint32_t>(t), ty)) visit(t);
-    if (!sure) return;
-    run(p.sureLo, p.sureHi);
-    for (int32_t t = p.sureHi + 1; t <= p.hi; ++t)
-        if (tile_touched(width, height, fp.cx, fp.cy, fp.a, fp.b, fp.c, fp.cut, static_cast<uint32_t>(t), ty)) visit(t);
-}
-
-// One row: its count, first and last touched column, and whether its hits
-// are one run.
-struct RowCount {
-    uint32_t count;
-    int32_t first, last;
-    bool regular;
-};
-__device__ __forceinline__ RowCount row_count(const Footprint& fp, uint32_t r, uint32_t width, uint32_t height) {
-    RowCount rc{0, 0, -2, true};
-    auto add = [&](int32_t t0, int32_t t1) {
-        if (rc.count != 0 && t0 != rc.last + 1) rc.regular = false;
-        if (rc.count == 0) rc.first = t0;
-        rc.count += static_cast<uint32_t>(t1 - t0 + 1);
-        rc.last = t1;
-    };
-    row_walk(fp, fp.y0 + r, width, height, [&](int32_t t) { add(t, t); }, add);
-    return rc;
-}
-constexpr uint64_t kFlagAggregate = 1ull << 62;
-constexpr uint64_t kFlagInclusive = 2ull << 62;
-constexpr uint64_t kValueMask = (1ull << 62) - 1;
-constexpr uint32_t kSpinLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* sWarp, uint32_t* total) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, x, d);
-        if (lane >= d) x += o;
-    }
-    if (lane == 31) sWarp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kProjectThreads / 32 ? sWarp[lane] : 0;
-#pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, w, d);
-            if (lane >= d) w += o;
-        }
-        if (lane < kProjectThreads / 32) sWarp[lane] = w;
-    }
-    __syncthreads();
-    const uint32_t before = warp == 0 ? 0 : sWarp[warp - 1];
-    *total = sWarp[kProjectThreads / 32 - 1];
-    __syncthreads();
-    return before + x - v;
-}
-
-// The block's first pair in the frame: warp 0 publishes the block's total
-// and looks back 32 partitions at a time (lane l reads the status of
-// partition q - l); the nearest inclusive prefix ends the walk and the
-// aggregates up to it are summed across the warp. A partition in the window
-// that has published nothing yet makes the warp read the window again
-// (bounded: after kSpinLimit polls kErrTimeout is raised and the walk
-// ends). The frame's last partition writes the pair total to counters[1].
-// Called by warp 0 only; lane 0's result is the block's base.
-__device__ __forceinline__ unsigned long long frame_lookback(uint64_t* __restrict__ status, uint32_t g,
-                                                             uint32_t lastPartition, uint32_t blockTotal,
-                                                             uint32_t* __restrict__ counters,
-                                                             uint32_t* __restrict__ err) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint64_t prefix = 0;
-    if (lane == 0) {
-        cuda::atomic_ref<uint64_t, cuda::thread_scope_device> mine(status[g]);
-        mine.store((g == 0 ? kFlagInclusive : kFlagAggregate) | blockTotal, cuda::memory_order_relaxed);
-    }
-    if (g > 0) {
-        int64_t q = static_cast<int64_t>(g) - 1;
-        uint32_t spins = 0;
-        while (true) {
-            const int64_t idx = q - static_cast<int64_t>(lane);
-            uint64_t word = kFlagInclusive;   // before partition 0: an empty inclusive prefix
-            if (idx >= 0) {
-                cuda::atomic_ref<uint64_t, cuda::thread_scope_device> sref(status[idx]);
-                word = sref.load(cuda::memory_order_relaxed);
-            }
-            const uint32_t inclusive = __ballot_sync(0xFFFFFFFFu, (word & kFlagInclusive) != 0);
-            const uint32_t empty = __ballot_sync(0xFFFFFFFFu, (word & ~kValueMask) == 0);
-            const uint32_t first = inclusive != 0 ? static_cast<uint32_t>(__ffs(inclusive)) - 1u : 32u;
-            const uint32_t upTo = first < 32u ? (2u << first) - 1u : 0xFFFFFFFFu;   // lanes 0..first
-            if ((empty & upTo) != 0) {
-                if (++spins > kSpinLimit) {
-                    if (lane == 0) atomicOr(err, kErrTimeout);
-                    break;
-                }
-                __nanosleep(32);
-                continue;
-            }
-            uint64_t v = ((upTo >> lane) & 1u) ? (word & kValueMask) : 0ull;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-            prefix += v;
-            if (first < 32u) break;
-            q -= 32;
-        }
-        if (lane == 0) {
-            cuda::atomic_ref<uint64_t, cuda::thread_scope_device> mine(status[g]);
-            mine.store(kFlagInclusive | (prefix + blockTotal), cuda::memory_order_relaxed);
-        }
-    }
-    if (lane == 0 && g == lastPartition) {
-        const uint64_t all = prefix + blockTotal;
-        if (all > 0xFFFFFFFFull) atomicOr(err, kErrTooManyPairs);
-        counters[1] = static_cast<uint32_t>(all);
-    }
-    return prefix;
-}
-
-// The position of the r-th set bit (from 0, lowest first) of a 64-bit mask
-// that has more than r set bits: the half, then five halvings by population
-// count.
-__device__ __forceinline__ uint32_t nth_set_bit(unsigned long long m, uint32_t r) {
-    uint32_t w = static_cast<uint32_t>(m);
-    uint32_t base = 0;
-    const uint32_t lowCount = static_cast<uint32_t>(__popc(w));
-    if (r >= lowCount) {
-        r -= lowCount;
-        w = static_cast<uint32_t>(m >> 32);
-        base = 32;
-    }
-#pragma unroll
-    for (uint32_t width = 16; width > 0; width >>= 1) {
-        const uint32_t lowBits = w & ((1u << width) - 1u);
-        const uint32_t c = static_cast<uint32_t>(__popc(lowBits));
-        if (r >= c) {
-            r -= c;
-            w >>= width;
-            base += width;
-        } else {
-            w = lowBits;
-        }
-    }
-    return base;
-}
-
-// The same over a 128-bit mask (lo, hi) with more than r set bits.
-__device__ __forceinline__ uint32_t nth_set_bit128(unsigned long long lo, unsigned long long hi, uint32_t r) {
-    const uint32_t lowCount = static_cast<uint32_t>(__popcll(lo));
-    return r < lowCount ? nth_set_bit(lo, r) : 64u + nth_set_bit(hi, r - lowCount);
-}
-
-// Row and column of bit `bit` of a row-major mask of width w (w <= 128,
-// bit < 128): (bit + 1/2) / w in float lies at least 1/256 away from an
-// integer, far more than its rounding error, so the floor is exact.
-__device__ __forceinline__ void mask_bit_tile(uint32_t bit, uint32_t w, float invW, uint32_t& dx, uint32_t& dy) {
-    dy = static_cast<uint32_t>((static_cast<float>(bit) + 0.5f) * invW);
-    dx = bit - dy * w;
-}
-
 struct PairSink {
     unsigned long long* pairs;
     uint32_t* values;     // training, emit index as a sort value
@@ -781,12 +495,20 @@ __device__ __forceinline__ void emit_by_warp(bool mine, uint32_t area, const uin
 }
 
 
+// Single frames of up to kMaxBands x kMaxBands tiles: per slot its touched
+// tiles and its runs of them, and the frame's runs per tile row (rows.cu).
+struct RunOutputs {
+    uint2* counts;
+    uint32_t* bands;
+};
+static_assert(kMaxBands == kProjectThreads, "a thread a tile row");
+
 // kEmit: emit the pairs (offsets by look-back over the frame's partitions).
 // Otherwise stop after the records and counts, and write per slot the
 // depth word (depth key << 32 | slot) the depth sort orders and the two aux
 // words emit_pairs_kernel reads: the tile mask of a masked splat, else 1 when
 // a row of a large splat's hits is not one run.
-template <class Src, bool kEmit = true, bool kChained = false>
+template <class Src, bool kEmit = true, bool kChained = false, bool kRuns = false>
 __global__ void __launch_bounds__(kProjectThreads, 4)
 project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src src, TrainOutputs train,
                     uint32_t stageWords, uint32_t shVector,
@@ -797,7 +519,7 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
                     unsigned long long* __restrict__ auxOut = nullptr,
                     unsigned long long* __restrict__ depthWordsOut = nullptr,
                     uint32_t* __restrict__ depthDigits = nullptr, uint2* __restrict__ rowTable = nullptr,
-                    uint32_t rowCap = 0) {
+                    uint32_t rowCap = 0, RunOutputs runsOut = {nullptr, nullptr}) {
     chained_entry<kChained>();
     extern __shared__ __align__(16) uint32_t shStage[];
     __shared__ uint32_t sPart;
@@ -816,6 +538,10 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
     // Without emission: the block's counts of the depth keys' three bytes
     // (the depth sort's digits), added to depthDigits at the end.
     __shared__ uint32_t sDigits[kEmit ? 1 : 3 * 256];
+    // The block's runs per tile row: sBands counts masked splats' runs, and
+    // sBandSteps what the running count of larger splats' rows changes by.
+    __shared__ uint32_t sBands[kRuns ? kMaxBands : 1];
+    __shared__ uint32_t sBandSteps[kRuns ? kMaxBands + 1 : 1];
     uint32_t* err = counters + 2;
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
@@ -825,6 +551,10 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
     }
     if constexpr (!kEmit) {
         for (uint32_t k = tid; k < 3 * 256; k += kProjectThreads) sDigits[k] = 0;
+        if constexpr (kRuns) {
+            sBands[tid] = 0;
+            sBandSteps[tid] = 0;
+        }
     }
     __syncthreads();
     const FrameParams& f = sF;
@@ -1165,7 +895,41 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
             atomicAdd(&sDigits[256 + ((key >> 8) & 0xFFu)], 1u);
             atomicAdd(&sDigits[512 + (key >> 16)], 1u);
         }
+        if (kRuns && inRange) {
+            // A masked splat's runs; a larger one's tile rows (or, when a row
+            // is not one run, its rectangle's tiles).
+            uint32_t runs = 0;
+            if (touched != 0 && masked) {
+                const ulonglong2 starts = mask_run_starts(mask, maskHi, rw);
+                runs = static_cast<uint32_t>(__popcll(starts.x) + __popcll(starts.y));
+                const float invW = 1.0f / static_cast<float>(rw);
+                unsigned long long word = starts.x;
+                for (uint32_t half = 0; half < 2; ++half, word = starts.y) {
+                    for (; word != 0; word &= word - 1ull) {
+                        uint32_t dx, dy;
+                        mask_bit_tile(64u * half + static_cast<uint32_t>(__ffsll(static_cast<long long>(word))) - 1u, rw,
+                                      invW, dx, dy);
+                        atomicAdd(&sBands[rect.y + dy], 1u);
+                    }
+                }
+            } else if (touched != 0) {
+                const uint32_t aRow = irregular ? rw : 1u;
+                runs = aRow * rh;
+                atomicAdd(&sBandSteps[rect.y], aRow);
+                atomicSub(&sBandSteps[rect.y + rh], aRow);
+            }
+            runsOut.counts[record] = make_uint2(touched, runs);
+        }
         __syncthreads();
+        if constexpr (kRuns) {
+            uint32_t v = sBands[tid];
+            if (anyBig) {
+                uint32_t all;
+                const uint32_t own = sBandSteps[tid];
+                v += block_exclusive_scan(own, sScan, &all) + own;
+            }
+            if (v != 0) atomicAdd(runsOut.bands + tid, v);
+        }
         for (uint32_t k = tid; k < 3 * 256; k += kProjectThreads) {
             const uint32_t v = sDigits[k];
             if (v != 0 && depthDigits != nullptr) atomicAdd(depthDigits + k, v);
@@ -1470,22 +1234,26 @@ template <class Src>
 cudaError_t launch_only(const FrameParams& f, const Src& src, bool stage, ProjRecord* proj, uint4* rects,
                         uint32_t* touched, uint32_t* keys, uint32_t* counters, uint32_t* ticket, uint64_t* aux,
                         uint64_t* depthWords, uint32_t* depthDigits, uint2* rowTable, uint32_t rowCap,
-                        cudaStream_t stream) {
+                        uint2* runCounts, uint32_t* bands, cudaStream_t stream) {
     const uint32_t stageWords = stage ? f.shWords : 0u;
     const uint32_t shVector = (reinterpret_cast<uintptr_t>(src.sh) & 15u) == 0 ? 1u : 0u;
     const size_t smem = stage ? size_t{kProjectThreads} * f.shWords * 4 : 0;
-    for (auto kernel : {project_emit_kernel<Src, false, true>, project_emit_kernel<Src, false, false>}) {
+    const bool runs = runCounts != nullptr;
+    const auto chained = runs ? project_emit_kernel<Src, false, true, true> : project_emit_kernel<Src, false, true, false>;
+    const auto plain = runs ? project_emit_kernel<Src, false, false, true> : project_emit_kernel<Src, false, false, false>;
+    for (auto kernel : {chained, plain}) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(std::max<size_t>(smem, 1)));
         if (e != cudaSuccess) return e;
     }
     const uint32_t blocks = project_partitions(f.count);
-    return launch_chained(project_emit_kernel<Src, false, true>, project_emit_kernel<Src, false, false>, dim3(blocks), dim3(kProjectThreads), smem, stream, f,
+    return launch_chained(chained, plain, dim3(blocks), dim3(kProjectThreads), smem, stream, f,
                           static_cast<const FrameParams*>(nullptr), src, TrainOutputs{nullptr, nullptr, nullptr},
                           stageWords, shVector, proj, rects, touched, keys, counters,
                           static_cast<uint64_t*>(nullptr), ticket, 0u, 0u, 0u, static_cast<unsigned long long*>(nullptr),
                           0u, reinterpret_cast<unsigned long long*>(aux),
-                          reinterpret_cast<unsigned long long*>(depthWords), depthDigits, rowTable, rowCap);
+                          reinterpret_cast<unsigned long long*>(depthWords), depthDigits, rowTable, rowCap,
+                          RunOutputs{runCounts, bands});
 }
 
 }  // namespace
@@ -1538,25 +1306,25 @@ cudaError_t launch_project_only(const FrameParams& f, const float4* positions, c
                                 const float* filter3d, ProjRecord* proj, uint4* rects, uint32_t* touched,
                                 uint32_t* keys, uint32_t* counters, uint32_t* ticket, uint64_t* aux,
                                 uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream) {
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream) {
     if (f.count == 0) return cudaSuccess;
     const uint32_t rpc = f.restPerColour;
     const uint32_t stored = rpc >= 15 ? 3u : rpc >= 8 ? 2u : rpc >= 3 ? 1u : 0u;
     const bool stage = std::min(stored, f.shLimit) > 0 && f.shWords > 0;
     return launch_only(f, PackedSource{positions, shape, sh, filter3d}, stage, proj, rects, touched, keys, counters,
-                       ticket, aux, depthWords, depthDigits, rowTable, rowCap, stream);
+                       ticket, aux, depthWords, depthDigits, rowTable, rowCap, runCounts, bands, stream);
 }
 
 cudaError_t launch_project_points_only(const FrameParams& f, const float4* positions, const uint32_t* colours,
                                        const lrt_point_style& style, ProjRecord* proj, uint4* rects, uint32_t* touched,
                                        uint32_t* keys, uint32_t* counters, uint32_t* ticket, uint64_t* aux,
                                        uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream) {
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream) {
     if (f.count == 0) return cudaSuccess;
     PointSource src{positions, reinterpret_cast<const uint2*>(colours), nullptr, style.size_mode, style.size,
                     style.constant_colour, {style.colour[0], style.colour[1], style.colour[2]}};
     return launch_only(f, src, false, proj, rects, touched, keys, counters, ticket, aux, depthWords, depthDigits,
-                       rowTable, rowCap, stream);
+                       rowTable, rowCap, runCounts, bands, stream);
 }
 
 cudaError_t launch_emit_sorted(const uint64_t* sortedWords, uint32_t n, const ProjRecord* proj, const uint4* rects,
@@ -1583,12 +1351,12 @@ cudaError_t launch_project_only_train(const FrameParams& f, const float* means, 
                                       const float* quats, const float* logits, const uint16_t* sh, ProjRecord* proj,
                                       uint4* rects, uint32_t* touched, uint32_t* keys, uint32_t* counters,
                                       uint32_t* ticket, uint64_t* aux, uint64_t* depthWords, uint32_t* depthDigits,
-                                uint2* rowTable, uint32_t rowCap, cudaStream_t stream) {
+                                uint2* rowTable, uint32_t rowCap, uint2* runCounts, uint32_t* bands, cudaStream_t stream) {
     if (f.count == 0) return cudaSuccess;
     // The DC triple is read from the staged row too, so it is always staged.
     return launch_only(f, RawSource{means, logScales, quats, logits, reinterpret_cast<const uint32_t*>(sh)}, true,
                        proj, rects, touched, keys, counters, ticket, aux, depthWords, depthDigits, rowTable, rowCap,
-                       stream);
+                       runCounts, bands, stream);
 }
 
 }  // namespace lrt

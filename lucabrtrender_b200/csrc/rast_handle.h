@@ -38,6 +38,9 @@ struct lrt_rast {
     DeviceBuffer algoKeysAlt, algoValsAlt;               // lrt_radix_sort's ping-pong buffers
     DeviceBuffer depthWords, depthWordsAlt, splatAux;    // per slot: depth words (two-step frames), aux words
     DeviceBuffer rowTable;                               // large splats' rows (first column, count)
+    DeviceBuffer runCounts, runs, runEmit, rowScratch;   // rows.cu: per slot, per run (and its first emit index), scratch
+    DeviceBuffer pairSlots, pairEmit;                    // rows.cu: every tile's slots (and, training, emit indices)
+    const uint32_t* debugLow = nullptr;                  // what the last frame's pair words hold below the tile (rows.cu)
     uint32_t rowCap = 0;                                 // its entries
     lrt::SortFault sortFault;                            // lrt_radix_sort's planted fault (tests only)
     DeviceBuffer filterCameras, filterScratch;           // lrt_rast_filter3d's cameras and lowest rate
@@ -47,6 +50,7 @@ struct lrt_rast {
     // counts copied to the host; ev[7..9]: the training backward's times.
     cudaEvent_t ev[10] = {};
     uint32_t splatCap = 0, pairCap = 0, tileCap = 0;
+    uint32_t seenPairs = 0, seenSlots = 0;   // the last single frame whose counts were read: its pairs and splats
     lrt_debug_view debug{};
     // Training: what the backward pass needs from its forward.
     DeviceBuffer pairValues, pairValuesAlt, pairOffsets, pixState, pixLast, partials;
@@ -80,6 +84,7 @@ struct lrt_rast {
     uint32_t* ringHostDev = nullptr;            // the device's address of ringHost
     cudaEvent_t ringEvent[kRing] = {};
     uint32_t ringCap[kRing] = {};               // the pair capacity each frame ran with
+    uint32_t ringSlots[kRing] = {};             // and its splats
     uint64_t ringHead = 0, ringTail = 0;        // next slot to fill; oldest slot not read
     bool plainSized = false;                    // a plain frame of this shape has run with a wait
     uint32_t plainSlots = 0, plainWidth = 0, plainHeight = 0, plainSeenPairs = 0;
@@ -135,6 +140,7 @@ namespace {
 using lrt::BlendParams;
 using lrt::FrameParams;
 using lrt::ProjRecord;
+using lrt::RowFrame;
 
 inline int fail(lrt_rast* r, int code, const std::string& message) {
     if (r != nullptr) r->error = message;

@@ -65,6 +65,7 @@ void lrt_rast_destroy(lrt_rast* r) {
     for (DeviceBuffer* b : {&r->proj, &r->rects, &r->touched, &r->keys, &r->pairs, &r->pairsAlt,
                             &r->ranges, &r->scanScratch, &r->sortScratch, &r->counters, &r->algoKeysAlt,
                             &r->algoValsAlt, &r->depthWords, &r->depthWordsAlt, &r->splatAux, &r->rowTable,
+                            &r->runCounts, &r->runs, &r->runEmit, &r->rowScratch, &r->pairSlots, &r->pairEmit,
                             &r->pairValues, &r->pairValuesAlt, &r->pairOffsets, &r->pixState, &r->pixLast, &r->partials, &r->metricScratch, &r->lossScratch, &r->trainBatchGrad,
                             &r->trainBatchViews, &r->trainBatchLoss, &r->lodBuild.globals,
                             &r->lodBuild.partial, &r->lodBuild.keys, &r->lodBuild.keysAlt, &r->lodBuild.order,
@@ -145,9 +146,25 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     const uint32_t tiles = tilesX * tilesY;
     const uint32_t tileBits = bits_for(tiles);
     // A frame takes the reference's two sorts: the projection alone, a sort
-    // of the slots' depth words, the pairs emitted in depth order as
-    // tile << 32 | slot (or emit index), and a stable sort of those on the tile
-    // bits (TileRasterizer.cpp:401-457).
+    // of the slots' depth words, the pairs in depth order, and a stable sort
+    // of those on the tile (TileRasterizer.cpp:401-457). The second sort is
+    // either one of the pairs as words tile << 32 | slot (or emit index) on
+    // their tile bits, or, where a splat touches many tiles, one of the
+    // splats' runs of tiles on their tile row, spread over the row's tiles
+    // (rows.cu: frames of at most 256 tiles a side).
+    // The line between them lies where both were measured alike, projection
+    // to ranges in ms, words against runs, by pairs a splat and pairs: 4.3 and
+    // 4.2M 0.265 / 0.267, 6.8 and 6.6M 0.347 / 0.320, 21 and 20M 0.757 /
+    // 0.573 (1M splats, 1080p); 7.3 and 2.1M 0.162 / 0.156, 12.5 and 3.6M
+    // 0.211 / 0.180 (300k, 1366x768); 13.6 and 1.3M 0.122 / 0.119, 7 and 0.7M
+    // 0.092 / 0.103 (100k, 512x512); 160 and 156M 3.69 / 1.83 (1M, 4K). The
+    // counts are those of the last frame of as many splats that was read.
+    constexpr uint32_t kRunsMinPairs = 1u << 21, kRunsMinPerSplat = 6;
+    const bool rowsAllowed = tilesX <= lrt::kMaxBands && tilesY <= lrt::kMaxBands;
+    auto runs_pay = [&](uint32_t pairCount) {
+        return rowsAllowed && pairCount >= kRunsMinPairs && pairCount / kRunsMinPerSplat >= slots;
+    };
+    bool byRows = r->seenSlots == slots && runs_pay(r->seenPairs);
 
     // Buffers (TileRasterizer.cpp:105-177).
     if (slots > r->splatCap) {
@@ -176,7 +193,9 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     // sort), counted by the kernels that write the keys.
     const size_t ticketsEnd = lrt::project_status_bytes(static_cast<uint32_t>(partitions)) + size_t{launches + 1} * 4;
     const size_t digitsAt = (ticketsEnd + 15) & ~size_t{15};
-    const size_t statusBytes = digitsAt + 5 * 256 * 4;
+    const size_t bandsAt = digitsAt + 5 * 256 * 4;
+    const size_t rowsAt = bandsAt + lrt::kMaxBands * 4;
+    const size_t statusBytes = rowsAllowed ? rowsAt + lrt::row_zeroed_bytes(slots) : bandsAt;
     LRT_CUDA(r, ensure(r->scanScratch, std::max<size_t>(statusBytes, 16)), "projection scratch");
     if (tiles > r->tileCap) {
         LRT_CUDA(r, ensure(r->ranges, size_t{tiles} * 8), "tile ranges");
@@ -196,6 +215,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                                                     lrt::project_status_bytes(static_cast<uint32_t>(partitions)));
     uint32_t* depthDigits = reinterpret_cast<uint32_t*>(static_cast<char*>(r->scanScratch.ptr) + digitsAt);
     uint32_t* tileDigits = depthDigits + 3 * 256;
+    uint32_t* bands = reinterpret_cast<uint32_t*>(static_cast<char*>(r->scanScratch.ptr) + bandsAt);
     const uint32_t tilePasses = (tileBits + 7) / 8 <= 2 ? (tileBits + 7) / 8 : 0u;
     const uint32_t lastPartition = partitions > 0 ? static_cast<uint32_t>(partitions - 1) : 0u;
     uint32_t visible = 0, pairs = 0, statusBits = 0;
@@ -220,29 +240,50 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     const bool lowIsEmit = train && !valuesAsked;
     bp.slotBits = 32;
     bp.tileShift = 32;
+    bp.pairShift = 1;
+    uint32_t* emitSlot = nullptr;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        LRT_CUDA(r, ensure(r->pairs, size_t{r->pairCap} * 8), "pairs");
-        LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * 8), "pairs");
-        if (train) {
-            LRT_CUDA(r, ensure(r->pairValues, size_t{r->pairCap} * 4), "pair values");
-            if (!lowIsEmit) LRT_CUDA(r, ensure(r->pairValuesAlt, size_t{r->pairCap} * 4), "pair values");
+        RowFrame rows{};
+        if (byRows) {
+            // A splat has a run where it has pairs, but for the empty rows at
+            // the ends of a few large ones' rectangles.
+            rows.runCap = static_cast<uint32_t>(
+                std::min<uint64_t>(uint64_t{r->pairCap} + r->pairCap / 4 + 1024, 0xFFFFF000ull));
+            rows.pairCap = r->pairCap;
+            LRT_CUDA(r, ensure(r->runCounts, size_t{r->splatCap} * sizeof(uint2)), "run counts");
+            LRT_CUDA(r, ensure(r->runs, size_t{rows.runCap} * 8), "runs");
+            LRT_CUDA(r, ensure(r->pairSlots, size_t{r->pairCap} * 4), "pairs");
+            LRT_CUDA(r, ensure(r->rowScratch, lrt::row_scratch_bytes(slots, rows.runCap, tilesX)), "row scratch");
+            if (train) {
+                LRT_CUDA(r, ensure(r->runEmit, size_t{rows.runCap} * 4), "runs");
+                LRT_CUDA(r, ensure(r->pairEmit, size_t{r->pairCap} * 4), "pairs");
+            }
+        } else {
+            LRT_CUDA(r, ensure(r->pairs, size_t{r->pairCap} * 8), "pairs");
+            LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * 8), "pairs");
+            if (train) {
+                LRT_CUDA(r, ensure(r->pairValues, size_t{r->pairCap} * 4), "pair values");
+                if (!lowIsEmit) LRT_CUDA(r, ensure(r->pairValuesAlt, size_t{r->pairCap} * 4), "pair values");
+            }
         }
         // The two sorts' scratch side by side, so that one launch clears it
         // with the counters, the projection's scratch and the tile ranges.
         const size_t depthScratch = lrt::sort_scratch_bytes(slots, 24);
         const size_t tileScratchAt = (depthScratch + 255) & ~size_t{255};
-        const size_t tileScratch = lrt::sort_scratch_bytes(r->pairCap, tileBits);
+        const size_t tileScratch = byRows ? 0 : lrt::sort_scratch_bytes(r->pairCap, tileBits);
         LRT_CUDA(r, ensure(r->sortScratch, tileScratchAt + tileScratch), "sort scratch");
         void* tileSortScratch = static_cast<char*>(r->sortScratch.ptr) + tileScratchAt;
-        const lrt::ZeroRegion clear[] = {{counters, 16},
+        const lrt::ZeroRegion clear[] = {{counters, 32},
                                          {r->scanScratch.ptr, statusBytes},
                                          {r->sortScratch.ptr, depthScratch},
                                          {tileSortScratch, tileScratch},
                                          {r->ranges.ptr, size_t{tiles} * sizeof(uint2)}};
         LRT_CUDA(r, lrt::launch_zero_regions(clear, 5, stream), "frame scratch");
         uint64_t* pairBuf = static_cast<uint64_t*>(r->pairs.ptr);
-        uint32_t* valueBuf = train && !lowIsEmit ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
-        uint32_t* emitSlot = train && lowIsEmit ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
+        uint32_t* valueBuf = train && !lowIsEmit && !byRows ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
+        emitSlot = train && lowIsEmit && !byRows ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
+        uint2* runCounts = byRows ? static_cast<uint2*>(r->runCounts.ptr) : nullptr;
+        uint32_t* bandsOut = byRows ? bands : nullptr;
 
         // --- project, count -------------------------------------------------------
         LRT_CUDA(r, cudaEventRecord(r->ev[0], stream), "event");
@@ -260,7 +301,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                              c.point->style, static_cast<ProjRecord*>(r->proj.ptr), static_cast<uint4*>(r->rects.ptr),
                              static_cast<uint32_t*>(r->touched.ptr), static_cast<uint32_t*>(r->keys.ptr), counters,
                              tickets + launch, aux, depthWords, depthDigits, static_cast<uint2*>(r->rowTable.ptr),
-                             r->rowCap, stream),
+                             r->rowCap, runCounts, bandsOut, stream),
                          "points");
             } else if (c.train != nullptr) {
                 const lrt_train_params& t = *c.train;
@@ -271,7 +312,8 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                              static_cast<const uint16_t*>(t.sh), static_cast<ProjRecord*>(r->proj.ptr),
                              static_cast<uint4*>(r->rects.ptr), static_cast<uint32_t*>(r->touched.ptr),
                              static_cast<uint32_t*>(r->keys.ptr), counters, tickets + launch, aux, depthWords,
-                             depthDigits, static_cast<uint2*>(r->rowTable.ptr), r->rowCap, stream),
+                             depthDigits, static_cast<uint2*>(r->rowTable.ptr), r->rowCap, runCounts, bandsOut,
+                             stream),
                          "project");
             } else {
                 LRT_CUDA(r,
@@ -281,7 +323,8 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                              static_cast<const float*>(c.packed->filter3d), static_cast<ProjRecord*>(r->proj.ptr),
                              static_cast<uint4*>(r->rects.ptr), static_cast<uint32_t*>(r->touched.ptr),
                              static_cast<uint32_t*>(r->keys.ptr), counters, tickets + launch, aux, depthWords,
-                             depthDigits, static_cast<uint2*>(r->rowTable.ptr), r->rowCap, stream),
+                             depthDigits, static_cast<uint2*>(r->rowTable.ptr), r->rowCap, runCounts, bandsOut,
+                             stream),
                          "project");
             }
             base += c.count;
@@ -297,30 +340,65 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                  "depth sort");
         const uint64_t* byDepth = depthInAlt ? static_cast<const uint64_t*>(r->depthWordsAlt.ptr) : depthWords;
         LRT_CUDA(r, cudaEventRecord(r->ev[4], stream), "event");
-        // --- pairs in depth order ----------------------------------------------------------
-        LRT_CUDA(r,
-                 lrt::launch_emit_sorted(byDepth, slots, static_cast<ProjRecord*>(r->proj.ptr),
-                                         static_cast<uint4*>(r->rects.ptr), static_cast<uint32_t*>(r->touched.ptr),
-                                         aux, s->width, s->height, tilesX, counters, status, tickets + launches,
-                                         static_cast<uint32_t*>(r->pairOffsets.ptr), pairBuf, r->pairCap,
-                                         tilePasses != 0 ? tileDigits : nullptr, tilePasses,
-                                         static_cast<const uint2*>(r->rowTable.ptr), stream, valueBuf, emitSlot),
-                 "emit");
-        LRT_CUDA(r, cudaEventRecord(r->ev[5], stream), "event");
-        // --- stable sort on the tile bits + ranges -------------------------------------------
-        bool inAlt = false;
-        LRT_CUDA(r,
-                 lrt::launch_sort_u64(pairBuf, static_cast<uint64_t*>(r->pairsAlt.ptr), valueBuf,
-                                      valueBuf != nullptr ? static_cast<uint32_t*>(r->pairValuesAlt.ptr) : nullptr,
-                                      counters + 1, r->pairCap, 32, tileBits, tileSortScratch, err, &inAlt, stream,
-                                      nullptr, tilePasses != 0 ? tileDigits : nullptr, true),
-                 "tile sort");
-        sorted = inAlt ? static_cast<uint64_t*>(r->pairsAlt.ptr) : pairBuf;
-        if (valueBuf != nullptr) sortedValues = inAlt ? static_cast<uint32_t*>(r->pairValuesAlt.ptr) : valueBuf;
-        LRT_CUDA(r,
-                 lrt::launch_ranges(sorted, counters + 1, r->pairCap, 32, static_cast<uint2*>(r->ranges.ptr), tiles,
-                                    stream, true),
-                 "ranges");
+        if (byRows) {
+            // --- the splats' runs of tiles, sorted by tile row ------------------------
+            rows.sortedWords = byDepth;
+            rows.slots = slots;
+            rows.width = s->width;
+            rows.height = s->height;
+            rows.tilesX = tilesX;
+            rows.tilesY = tilesY;
+            rows.proj = static_cast<ProjRecord*>(r->proj.ptr);
+            rows.rects = static_cast<uint4*>(r->rects.ptr);
+            rows.aux = aux;
+            rows.rowTable = static_cast<const uint2*>(r->rowTable.ptr);
+            rows.runCounts = runCounts;
+            rows.bands = bands;
+            rows.counters = counters;
+            rows.pairOffsets = train ? static_cast<uint32_t*>(r->pairOffsets.ptr) : nullptr;
+            rows.runs = static_cast<uint64_t*>(r->runs.ptr);
+            rows.runEmit = train ? static_cast<uint32_t*>(r->runEmit.ptr) : nullptr;
+            rows.pairSlots = static_cast<uint32_t*>(r->pairSlots.ptr);
+            rows.pairEmit = train ? static_cast<uint32_t*>(r->pairEmit.ptr) : nullptr;
+            rows.ranges = static_cast<uint2*>(r->ranges.ptr);
+            rows.zeroed = static_cast<char*>(r->scanScratch.ptr) + rowsAt;
+            rows.scratch = r->rowScratch.ptr;
+            LRT_CUDA(r, lrt::launch_row_runs(rows, stream), "runs");
+            LRT_CUDA(r, cudaEventRecord(r->ev[5], stream), "event");
+            // --- every tile's slots in depth order, and its range -----------------------
+            LRT_CUDA(r, lrt::launch_row_pairs(rows, stream), "pairs");
+            bp.pairShift = 0;
+            sorted = reinterpret_cast<const uint64_t*>(rows.pairSlots);
+            sortedValues = rows.pairEmit;
+            r->debugLow = lowIsEmit ? rows.pairEmit : rows.pairSlots;
+        } else {
+            bp.pairShift = 1;
+            // --- pairs in depth order ----------------------------------------------------------
+            LRT_CUDA(r,
+                     lrt::launch_emit_sorted(byDepth, slots, static_cast<ProjRecord*>(r->proj.ptr),
+                                             static_cast<uint4*>(r->rects.ptr), static_cast<uint32_t*>(r->touched.ptr),
+                                             aux, s->width, s->height, tilesX, counters, status, tickets + launches,
+                                             static_cast<uint32_t*>(r->pairOffsets.ptr), pairBuf, r->pairCap,
+                                             tilePasses != 0 ? tileDigits : nullptr, tilePasses,
+                                             static_cast<const uint2*>(r->rowTable.ptr), stream, valueBuf, emitSlot),
+                     "emit");
+            LRT_CUDA(r, cudaEventRecord(r->ev[5], stream), "event");
+            // --- stable sort on the tile bits + ranges -------------------------------------------
+            bool inAlt = false;
+            LRT_CUDA(r,
+                     lrt::launch_sort_u64(pairBuf, static_cast<uint64_t*>(r->pairsAlt.ptr), valueBuf,
+                                          valueBuf != nullptr ? static_cast<uint32_t*>(r->pairValuesAlt.ptr) : nullptr,
+                                          counters + 1, r->pairCap, 32, tileBits, tileSortScratch, err, &inAlt, stream,
+                                          nullptr, tilePasses != 0 ? tileDigits : nullptr, true),
+                     "tile sort");
+            sorted = inAlt ? static_cast<uint64_t*>(r->pairsAlt.ptr) : pairBuf;
+            if (valueBuf != nullptr) sortedValues = inAlt ? static_cast<uint32_t*>(r->pairValuesAlt.ptr) : valueBuf;
+            LRT_CUDA(r,
+                     lrt::launch_ranges(sorted, counters + 1, r->pairCap, 32, static_cast<uint2*>(r->ranges.ptr), tiles,
+                                        stream, true),
+                     "ranges");
+            r->debugLow = nullptr;
+        }
         // The blend takes the tiles busiest first (the composite blend keeps
         // index order).
         uint32_t* tileOrder = composite ? nullptr : static_cast<uint32_t*>(r->tileOrder.ptr);
@@ -364,6 +442,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         if (ring) {
             LRT_CUDA(r, cudaEventRecord(r->ringEvent[slot], stream), "event");
             r->ringCap[slot] = r->pairCap;
+            r->ringSlots[slot] = slots;
             r->ringHead += 1;
         }
         if (deferred) {
@@ -371,7 +450,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             r->debug.rects = r->rects.ptr;
             r->debug.touched = r->touched.ptr;
             r->debug.depth_keys = r->keys.ptr;
-            r->debug.pairs = sorted;
+            r->debug.pairs = byRows ? nullptr : sorted;
             r->debug.ranges = r->ranges.ptr;
             r->debug.slots = slots;
             r->debug.tiles = tiles;
@@ -402,9 +481,13 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         visible = r->hostCounters[0];
         pairs = r->hostCounters[1];
         statusBits = r->hostCounters[2];
+        r->seenPairs = pairs;
+        r->seenSlots = slots;
         if (statusBits & lrt::kErrTooManyPairs) return fail(r, LRT_UNSUPPORTED, "more than 2^32 pairs in one frame");
-        if (pairs <= r->pairCap) break;
-        r->pairCap = grow(r->pairCap, pairs);   // draw again with room for every pair
+        if (pairs <= r->pairCap && (statusBits & lrt::kErrOverflow) == 0) break;
+        // Draw again with room for every pair (and every run).
+        r->pairCap = grow(r->pairCap, std::max(pairs, r->pairCap + 1));
+        byRows = runs_pay(pairs);
         statusBits &= ~lrt::kErrOverflow;
     }
     // Rows the frame's large splats asked for beyond the row table: the next
@@ -415,7 +498,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     r->debug.rects = r->rects.ptr;
     r->debug.touched = r->touched.ptr;
     r->debug.depth_keys = r->keys.ptr;
-    r->debug.pairs = sorted;
+    r->debug.pairs = byRows ? nullptr : sorted;
     r->debug.ranges = r->ranges.ptr;
     r->debug.slots = slots;
     r->debug.pairs_count = pairs;
@@ -431,7 +514,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         r->trainBlend = bp;
         r->trainSorted = sorted;
         r->trainSortedValues = sortedValues;
-        r->trainEmitSlot = lowIsEmit ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
+        r->trainEmitSlot = emitSlot;
         r->trainPairs = pairs;
         r->trainReady = true;
     }
@@ -503,9 +586,11 @@ bool read_oldest(lrt_rast* r, bool wait) {
     r->asyncVisible = c[0];
     r->asyncPairs = c[1];
     r->plainSeenPairs = c[1];
-    if (c[1] > r->ringCap[slot] || (c[2] & lrt::kErrTooManyPairs) != 0) {
+    r->seenPairs = c[1];
+    r->seenSlots = r->ringSlots[slot];
+    if (c[1] > r->ringCap[slot] || (c[2] & (lrt::kErrTooManyPairs | lrt::kErrOverflow)) != 0) {
         r->asyncOverflows += 1;
-        r->pairCap = std::max(r->pairCap, grow(r->pairCap, c[1]));
+        r->pairCap = std::max(r->pairCap, grow(r->pairCap, std::max(c[1], r->ringCap[slot] + 1)));
     }
     if (c[2] & lrt::kErrTimeout) r->asyncTimeouts += 1;
     r->debug.visible = c[0];
@@ -923,10 +1008,12 @@ static int settle_pending_frame(lrt_rast* r) {
     const uint32_t pairs = r->hostCounters[1], status = r->hostCounters[2];
     r->trainPairs = std::min(pairs, r->pairCap);
     r->trainSeenPairs = pairs;
+    r->seenPairs = pairs;
+    r->seenSlots = r->trainParams.count;
     r->debug.pairs_count = std::min(pairs, r->pairCap);
     r->debug.visible = r->hostCounters[0];
-    if (pairs > r->pairCap) {
-        r->pairCap = grow(r->pairCap, pairs);
+    if (pairs > r->pairCap || (status & lrt::kErrOverflow) != 0) {
+        r->pairCap = grow(r->pairCap, std::max(pairs, r->pairCap + 1));
         r->trainReady = false;
         return fail(r, LRT_OVERFLOW, "the training forward emitted more pairs than its buffer held; "
                                      "the buffers are grown, run the step again");
@@ -1036,6 +1123,18 @@ int lrt_rast_debug_view(lrt_rast* r, lrt_debug_view* out) {
         if (code != LRT_OK) return code;
     }
     *out = r->debug;
+    if (r->debugLow != nullptr && out->pairs == nullptr && out->tiles != 0) {
+        // Frames made from runs keep every tile's slots, not pair words: they
+        // are put together here, where they are looked at.
+        DeviceScope scope(r->device);
+        LRT_CUDA(r, ensure(r->pairs, std::max<size_t>(size_t{out->pairs_count} * 8, 16)), "pair words");
+        LRT_CUDA(r,
+                 lrt::launch_pair_words(static_cast<const uint2*>(out->ranges), r->debugLow, out->tiles, out->pairs_count,
+                                        static_cast<uint64_t*>(r->pairs.ptr), nullptr),
+                 "pair words");
+        LRT_CUDA(r, cudaStreamSynchronize(nullptr), "pair words");
+        out->pairs = r->pairs.ptr;
+    }
     return LRT_OK;
 }
 
@@ -1163,6 +1262,7 @@ int enqueue_batch(lrt_rast* r, const std::vector<CloudDesc>& clouds, const lrt_v
     BlendParams bp{};
     bp.slotBits = slotBits;
     bp.tileShift = 24 + slotBits;
+    bp.pairShift = 1;
     bp.depthMode = s->depth_mode;
     bp.linearise = s->linearise ? 1u : 0u;
     bp.depthThreshold = s->depth_threshold;

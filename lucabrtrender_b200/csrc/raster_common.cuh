@@ -95,6 +95,9 @@ struct FrameParams {
 struct BlendParams {
     uint32_t width, height, tilesX, tilesY;
     uint32_t slotBits, tileShift;
+    // log2 of the 32-bit words a pair takes: 1 for pair words, 0 where only
+    // every tile's slots are kept (rows.cu).
+    uint32_t pairShift;
     uint32_t depthMode, linearise;
     float depthThreshold;
     float bg[4];
@@ -278,6 +281,19 @@ __device__ __forceinline__ uint32_t pack_halves(float a, float b) {
     if (isnan(a) || isnan(b)) return (float_to_half(a) & 0xFFFFu) | ((float_to_half(b) & 0xFFFFu) << 16);
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// The lanes of the warp holding the same digit d (0..255), from one ballot
+// per digit bit.
+__device__ __forceinline__ uint32_t match_digit(uint32_t d) {
+    uint32_t m = 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t b = 0; b < 8; ++b) {
+        const bool bit = ((d >> b) & 1u) != 0;
+        const uint32_t v = __ballot_sync(0xFFFFFFFFu, bit);
+        m &= bit ? v : ~v;
+    }
+    return m;
 }
 
 // Asynchronous global -> shared copies (cp.async): a thread issues all of its

@@ -88,19 +88,6 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
     return before + x - v;
 }
 
-// The lanes of the warp holding the same digit d (0..255), from one ballot
-// per digit bit.
-__device__ __forceinline__ uint32_t match_digit(uint32_t d) {
-    uint32_t m = 0xFFFFFFFFu;
-#pragma unroll
-    for (uint32_t b = 0; b < 8; ++b) {
-        const bool bit = ((d >> b) & 1u) != 0;
-        const uint32_t v = __ballot_sync(0xFFFFFFFFu, bit);
-        m &= bit ? v : ~v;
-    }
-    return m;
-}
-
 template <typename K>
 __device__ __forceinline__ uint32_t digit_of(K key, uint32_t shift) {
     return static_cast<uint32_t>(key >> shift) & 0xFFu;

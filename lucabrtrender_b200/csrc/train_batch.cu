@@ -210,6 +210,7 @@ int enqueue_step(lrt_rast* r, const StepArgs& a, const Layout& L, uint32_t cap, 
     BlendParams bp{};
     bp.slotBits = slotBits;
     bp.tileShift = 24 + slotBits;
+    bp.pairShift = 1;
     bp.depthMode = a.s->depth_mode;
     bp.linearise = a.s->linearise ? 1u : 0u;
     bp.depthThreshold = a.s->depth_threshold;
