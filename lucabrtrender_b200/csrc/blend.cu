@@ -138,6 +138,7 @@ struct CompositeShared {
 
 __device__ __forceinline__ float2 lower2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 upper2(float4 v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) < INFINITY; }
 
 // shaders/lrt/splat/splat_blend.slang:23-108 (splat-only entry, :110-114).
 // One block of 128 threads per 16x16 tile, two pixels a thread. The tile's
