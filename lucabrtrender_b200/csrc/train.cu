@@ -15,6 +15,8 @@ namespace lrt {
 namespace {
 
 constexpr uint32_t kThreads = 128;
+constexpr uint32_t kFrameBlocks = 7;   // resident blocks aimed at: one frame's pass
+constexpr uint32_t kViewsBlocks = 4;   // and a chunk of views'
 constexpr uint32_t kMaxChunkViews = 16;   // views one splat_backward_views launch takes
 constexpr uint32_t kGradStrideFloats = 12;  // floats per pair in the partials buffer
 constexpr float kC1 = 0.4886025119029199f;
@@ -98,11 +100,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // One view's gradients of splat i from its summed partials g: the per-view
 // means, log-scale, quaternion and logit gradients added into gm, gls, gq,
 // glog (which the caller zeroes), and the 48 SH gradients handed to
-// sink(q, value) in coefficient order.
+// sink(v, values) four at a time, v = 0..11, in coefficient order. shRow: the
+// splat's 48 fp16 coefficients in shared memory, eight a vector; vector v is
+// read (last) before sink(2 v) is called.
 template <class ShSink>
 __device__ __forceinline__ void view_grads(const FrameParams& f, uint32_t i, const float* __restrict__ means,
                                            const float* __restrict__ logScales, const float* __restrict__ quats,
-                                           const float* __restrict__ logits, const uint16_t* __restrict__ sh,
+                                           const float* __restrict__ logits, const float4* shRow,
                                            const float (&g)[9], float (&gm)[3], float (&gls)[3], float (&gq)[4],
                                            float& glog, ShSink&& sink) {
     const float gcx = g[0], gcy = g[1], gA = g[2], gB = g[3], gC = g[4], gAlpha = g[5];
@@ -165,62 +169,65 @@ __device__ __forceinline__ void view_grads(const FrameParams& f, uint32_t i, con
     const float QA = c / det, QB = -b / det, QC = a / det;
 
     // ---- colour ---------------------------------------------------------------
-    // The fp16 coefficients stay packed (24 words, read as six 16-byte
-    // vectors) and are unpacked where used; each basis function and its
-    // gradient is formed where it is used, in two passes over the 15 rest
-    // functions (the rest sum, then the gradients), so that no 48-value
+    // The fp16 coefficients are read from the staged row eight at a time, in
+    // two passes (the rest sum, then the gradients), and each basis function
+    // and its gradient is formed where it is used, so that no 48-value
     // arrays are held at once.
-    uint32_t cw[24];
-    {
-        const uint4* rv = reinterpret_cast<const uint4*>(sh + static_cast<size_t>(i) * 48);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const uint4 w4 = __ldg(rv + q);
-            cw[4 * q] = w4.x;
-            cw[4 * q + 1] = w4.y;
-            cw[4 * q + 2] = w4.z;
-            cw[4 * q + 3] = w4.w;
-        }
-    }
-    auto coef = [&](int q) { return (q & 1) != 0 ? high_half(cw[q >> 1]) : low_half(cw[q >> 1]); };
+    auto coef = [](const float4& w, int e) {
+        const uint32_t u = __float_as_uint(e < 2 ? w.x : e < 4 ? w.y : e < 6 ? w.z : w.w);
+        return (e & 1) != 0 ? high_half(u) : low_half(u);
+    };
     float vx = px - f.eye[0], vy = py - f.eye[1], vz = pz - f.eye[2];
     const float vl = sqrtf(vx * vx + vy * vy + vz * vz);
     const float dirx = vx / vl, diry = vy / vl, dirz = vz / vl;
     const uint32_t degree = min(3u, f.shLimit);   // basis functions above it are 0
     const int used = degree == 0 ? 0 : degree == 1 ? 3 : degree == 2 ? 8 : 15;
     constexpr float kSH0 = 0.28209479177387814f;
-    float rest[3] = {0.0f, 0.0f, 0.0f};
+    float rest[3] = {0.0f, 0.0f, 0.0f}, base[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int k = 0; k < 15; ++k) {
-        if (k < used) {
-            const float b = sh_basis_at(k, dirx, diry, dirz);
+    for (int v = 0; v < 6; ++v) {
+        const float4 w = shRow[v];
 #pragma unroll
-            for (int ch = 0; ch < 3; ++ch) rest[ch] += b * coef(3 + 3 * k + ch);
+        for (int e = 0; e < 8; ++e) {
+            const int q = 8 * v + e, k = (q - 3) / 3;
+            if (q < 3) {
+                base[q] = 0.5f + kSH0 * coef(w, e);
+            } else if (k < used) {
+                rest[(q - 3) % 3] += sh_basis_at(k, dirx, diry, dirz) * coef(w, e);
+            }
         }
     }
     // colour = max(base + rest, 0): no gradient where clamped. Basis
     // functions above the evaluated degree are 0, so their coefficients get 0.
     float gcol[3];
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
-        const float base = 0.5f + kSH0 * coef(ch);
-        gcol[ch] = base + rest[ch] > 0.0f ? g[6 + ch] : 0.0f;
-        sink(ch, kSH0 * gcol[ch]);
-    }
+    for (int ch = 0; ch < 3; ++ch) gcol[ch] = base[ch] + rest[ch] > 0.0f ? g[6 + ch] : 0.0f;
     float gdx = 0.0f, gdy = 0.0f, gdz = 0.0f;
+    float basis = 0.0f, bx = 0.0f, by = 0.0f, bz = 0.0f, cg = 0.0f;
+    float out[4];
 #pragma unroll
-    for (int k = 0; k < 15; ++k) {
-        float b = 0.0f, bx = 0.0f, by = 0.0f, bz = 0.0f;
-        if (k < used) sh_basis_grad_at(k, dirx, diry, dirz, b, bx, by, bz);
-        float cg = 0.0f;
+    for (int v = 0; v < 6; ++v) {
+        const float4 w = shRow[v];
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            sink(3 + 3 * k + ch, b * gcol[ch]);
-            cg += coef(3 + 3 * k + ch) * gcol[ch];
+        for (int e = 0; e < 8; ++e) {
+            const int q = 8 * v + e, k = (q - 3) / 3, ch = (q - 3) % 3;
+            if (q < 3) {
+                out[e & 3] = kSH0 * gcol[q];
+            } else {
+                if (ch == 0) {
+                    basis = bx = by = bz = cg = 0.0f;
+                    if (k < used) sh_basis_grad_at(k, dirx, diry, dirz, basis, bx, by, bz);
+                }
+                out[e & 3] = basis * gcol[ch];
+                cg += coef(w, e) * gcol[ch];
+                if (ch == 2) {
+                    gdx += cg * bx;
+                    gdy += cg * by;
+                    gdz += cg * bz;
+                }
+            }
+            if ((e & 3) == 3) sink(q >> 2, make_float4(out[0], out[1], out[2], out[3]));
         }
-        gdx += cg * bx;
-        gdy += cg * by;
-        gdz += cg * bz;
     }
     {   // dir = v / |v|, v = p - eye
         const float dotd = gdx * dirx + gdy * diry + gdz * dirz;
@@ -367,10 +374,71 @@ __device__ __forceinline__ void splat_partials(uint32_t count, uint32_t firstRaw
     nOut = n;
 }
 
+// ---- a warp's rows of SH gradients and coefficients in shared memory ----
+//
+// A splat's 48 SH gradients are one row of 13 vectors (48 floats and a
+// vector of padding: an odd pitch, so that 32 lanes' vectors at one place of
+// their rows meet no bank conflict, and neither do consecutive vectors).
+constexpr uint32_t kRowVectors = 13;
+constexpr uint32_t kShVectors = 6;   // vectors of a splat's 48 fp16 coefficients
+
+// The fp16 coefficients of the warp's `rows` splats from `src` to rows of
+// `pitch` vectors starting at `dst`, by 16-byte asynchronous copies.
+__device__ __forceinline__ void stage_sh(float4* dst, uint32_t pitch, const uint16_t* src, uint32_t rows, uint32_t lane) {
+    const float4* from = reinterpret_cast<const float4*>(src);
+#pragma unroll
+    for (uint32_t j = 0; j < kShVectors; ++j) {
+        const uint32_t v = lane + 32 * j;
+        if (v < rows * kShVectors) cp_async16(dst + (v / kShVectors) * pitch + v % kShVectors, from + v);
+    }
+}
+
+// A warp's `floats` floats from shared memory to consecutive addresses.
+__device__ __forceinline__ void copy_out(float* dst, const float* src, uint32_t floats, uint32_t lane) {
+    for (uint32_t k = lane; k < floats; k += 32) dst[k] = src[k];
+}
+
+// The warp's gradients to memory, consecutive lanes on consecutive addresses:
+// its rows of SH gradients, then the others by way of the rows' place.
+__device__ __forceinline__ void write_warp(float4* rows, uint32_t n, size_t first, uint32_t lane, const float (&gm)[3],
+                                           const float (&gls)[3], const float (&gq)[4], float glog, float* gMeans,
+                                           float* gLogScales, float* gQuats, float* gLogits, float* gSh) {
+    __syncwarp();
+    float4* out = reinterpret_cast<float4*>(gSh + first * 48);
+#pragma unroll
+    for (uint32_t j = 0; j < 12; ++j) {
+        const uint32_t v = lane + 32 * j;
+        if (v < n * 12) out[v] = rows[(v / 12) * kRowVectors + v % 12];
+    }
+    __syncwarp();
+    float* flat = reinterpret_cast<float*>(rows);
+#pragma unroll
+    for (uint32_t k = 0; k < 3; ++k) {
+        flat[3 * lane + k] = gm[k];
+        flat[96 + 3 * lane + k] = gls[k];
+    }
+    reinterpret_cast<float4*>(flat + 192)[lane] = make_float4(gq[0], gq[1], gq[2], gq[3]);
+    __syncwarp();
+    copy_out(gMeans + 3 * first, flat, 3 * n, lane);
+    copy_out(gLogScales + 3 * first, flat + 96, 3 * n, lane);
+    copy_out(gQuats + 4 * first, flat + 192, 4 * n, lane);
+    if (lane < n) gLogits[first + lane] = glog;
+}
+
 // One frame: every splat's gradients written (zero for a splat the frame
-// does not touch).
+// does not touch). A warp works on 32 consecutive splats with no barrier
+// beyond its own: their coefficients are copied into the ends of the rows
+// that the SH gradients then fill (the gradients' end never passes the
+// coefficients still to be read: 32 v + 32 <= 112 + 16 (v + 1) bytes for
+// v < 6), so a block's 26 KB hold both.
+// Bound by the latency of count -> partials -> chain rule, with 600 MB to
+// move at 1M splats, 1080p (0.093 ms at the copy rate): seven blocks an SM,
+// the coefficients in shared memory instead of 24 registers, and whole-warp
+// stores of consecutive addresses (a thread's own row a vector at a time
+// touched 32 sectors a store): 0.201 -> 0.169 ms (2.9 -> 3.6 TB/s); six
+// blocks 0.175, eight (64 registers) 0.197.
 template <bool kChained>
-__global__ void __launch_bounds__(kThreads, 5)
+__global__ void __launch_bounds__(kThreads, kFrameBlocks)
 splat_backward_kernel(FrameParams f, const float* __restrict__ means, const float* __restrict__ logScales,
                       const float* __restrict__ quats, const float* __restrict__ logits,
                       const uint16_t* __restrict__ sh, const uint32_t* __restrict__ touched,
@@ -378,62 +446,59 @@ splat_backward_kernel(FrameParams f, const float* __restrict__ means, const floa
                       uint32_t partialPairs, float* __restrict__ gMeans, float* __restrict__ gLogScales,
                       float* __restrict__ gQuats, float* __restrict__ gLogits, float* __restrict__ gSh) {
     chained_entry<kChained>();
-    __shared__ float sGsh[48][kThreads];
+    __shared__ float4 sRows[kThreads * kRowVectors];
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t first = i - lane;   // the warp's first splat
+    if (first >= f.count) return;
+    const uint32_t rows = min(32u, f.count - first);
     const bool live = i < f.count;
     const uint32_t slot = f.base + i;
-    // The parameters and SH row are read only after the partials are summed;
-    // ask for them now (into L2, no registers held), so their DRAM latency
-    // overlaps the count, offset and partial loads that each wait on the last.
+    float4* warpRows = sRows + (threadIdx.x - lane) * kRowVectors;
+    float4* row = warpRows + lane * kRowVectors;
+    float4* coefficients = warpRows + (kRowVectors - kShVectors);
+    const uint32_t count = live ? touched[slot] : 0u;
+    const uint32_t firstRaw = live ? offsets[slot] : 0u;   // loaded beside the count, not after it
+    // The parameters are read only after the partials are summed; ask for
+    // them now (the harmonics into shared memory, the others into L2, no
+    // registers held), so their DRAM latency overlaps the count, offset and
+    // partial loads that each wait on the last.
+    stage_sh(coefficients, kRowVectors, sh + 48 * static_cast<size_t>(first), rows, lane);
     if (live) {
         prefetch_l2(means + 3 * static_cast<size_t>(i));
         prefetch_l2(logScales + 3 * static_cast<size_t>(i));
         prefetch_l2(quats + 4 * static_cast<size_t>(i));
         prefetch_l2(logits + i);
-        prefetch_l2(sh + 48 * static_cast<size_t>(i));
-        prefetch_l2(sh + 48 * static_cast<size_t>(i) + 40);
     }
     float g[9];
     uint32_t n = 0;
-    const uint32_t count = live ? touched[slot] : 0u;
-    const uint32_t firstRaw = live ? offsets[slot] : 0u;   // loaded beside the count, not after it
     splat_partials(count, firstRaw, lane, partials, partialPairs, g, n);
-    if (!live) return;
+    cp_async_wait_all();
+    __syncwarp();
     float gm[3] = {0, 0, 0}, gls[3] = {0, 0, 0}, gq[4] = {0, 0, 0, 0}, glog = 0.0f;
-    float* gshRow = gSh + static_cast<size_t>(i) * 48;
     if (n == 0) {
-        float4* out = reinterpret_cast<float4*>(gshRow);
 #pragma unroll
-        for (int q = 0; q < 12; ++q) out[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (uint32_t v = 0; v < 12; ++v) row[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     } else {
-        // The 48 SH gradients go through shared memory (a column per thread)
-        // rather than registers, then out as 16-byte stores.
-        view_grads(f, i, means, logScales, quats, logits, sh, g, gm, gls, gq, glog,
-                   [&](int q, float v) { sGsh[q][threadIdx.x] = v; });
-        float4* out = reinterpret_cast<float4*>(gshRow);
-#pragma unroll
-        for (int q = 0; q < 12; ++q)
-            out[q] = make_float4(sGsh[4 * q][threadIdx.x], sGsh[4 * q + 1][threadIdx.x], sGsh[4 * q + 2][threadIdx.x],
-                                 sGsh[4 * q + 3][threadIdx.x]);
+        view_grads(f, i, means, logScales, quats, logits, coefficients + lane * kRowVectors, g, gm, gls, gq, glog,
+                   [&](int v, const float4& x) { row[v] = x; });
     }
-    for (int k = 0; k < 3; ++k) {
-        gMeans[3 * i + k] = gm[k];
-        gLogScales[3 * i + k] = gls[k];
-    }
-    for (int k = 0; k < 4; ++k) gQuats[4 * i + k] = gq[k];
-    gLogits[i] = glog;
+    write_warp(warpRows, rows, first, lane, gm, gls, gq, glog, gMeans, gLogScales, gQuats, gLogits, gSh);
 }
 
 // A chunk of views in one pass. Per splat, view after view in order, the
 // view's gradients (view_grads, as above) are added to running sums -- the
-// 48 SH ones in shared memory, a column per thread -- and the sums written
-// once at the end, so the gradient buffers are read and written once a chunk
-// rather than once a view. The sums start from what the buffers hold when
-// `accumulate` is set (a batch's later chunks), else from zero: the same
-// float additions, in the same order, as a view-by-view pass adding each
-// view to the buffers. touched / offsets: one array of `count` per view.
-__global__ void __launch_bounds__(kThreads, 3)
+// 48 SH ones in the splat's row in shared memory, beside its coefficients,
+// which are read once for all views -- and the sums written once at the end,
+// so the gradient buffers are read and written once a chunk rather than once
+// a view. The sums start from what the buffers hold when `accumulate` is set
+// (a batch's later chunks), else from zero: the same float additions, in the
+// same order, as a view-by-view pass adding each view to the buffers.
+// touched / offsets: one array of `count` per view. 400k splats, 6 views:
+// 0.376 -> 0.335 ms at four blocks an SM (three 0.376, five 0.333).
+constexpr uint32_t kShPitch = 7;   // vectors from one row of coefficients to the next (odd, as above)
+
+__global__ void __launch_bounds__(kThreads, kViewsBlocks)
 splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t views, uint32_t count,
                             const float* __restrict__ means, const float* __restrict__ logScales,
                             const float* __restrict__ quats, const float* __restrict__ logits,
@@ -442,7 +507,8 @@ splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t vie
                             uint32_t partialPairs, float* __restrict__ gMeans, float* __restrict__ gLogScales,
                             float* __restrict__ gQuats, float* __restrict__ gLogits, float* __restrict__ gSh,
                             uint32_t accumulate) {
-    __shared__ float sAcc[48][kThreads];
+    __shared__ float4 sRows[kThreads * kRowVectors];
+    __shared__ float4 sSh[kThreads * kShPitch - 1];
     __shared__ FrameParams sF[kMaxChunkViews];
     {
         const uint32_t words = views * static_cast<uint32_t>(sizeof(FrameParams) / 4);
@@ -453,9 +519,13 @@ splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t vie
     const uint32_t tid = threadIdx.x;
     const uint32_t i = blockIdx.x * kThreads + tid;
     const uint32_t lane = tid & 31u;
+    const uint32_t first = i - lane;
+    const uint32_t rows = first < count ? min(32u, count - first) : 0u;
     const bool live = i < count;
     float am[3] = {0, 0, 0}, als[3] = {0, 0, 0}, aq[4] = {0, 0, 0, 0}, alog = 0.0f;
-    float4* shRow = reinterpret_cast<float4*>(gSh + static_cast<size_t>(i) * 48);
+    float4* warpRows = sRows + (tid - lane) * kRowVectors;
+    float4* row = warpRows + lane * kRowVectors;
+    if (rows != 0) stage_sh(sSh + (tid - lane) * kShPitch, kShPitch, sh + 48 * static_cast<size_t>(first), rows, lane);
     if (live && accumulate != 0) {
         for (int k = 0; k < 3; ++k) {
             am[k] = gMeans[3 * i + k];
@@ -463,19 +533,17 @@ splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t vie
         }
         for (int k = 0; k < 4; ++k) aq[k] = gQuats[4 * i + k];
         alog = gLogits[i];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) {
-            const float4 v = shRow[q];
-            sAcc[4 * q][tid] = v.x;
-            sAcc[4 * q + 1][tid] = v.y;
-            sAcc[4 * q + 2][tid] = v.z;
-            sAcc[4 * q + 3][tid] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 48; ++q) sAcc[q][tid] = 0.0f;
     }
+    const float4* held = reinterpret_cast<const float4*>(gSh + static_cast<size_t>(first) * 48);
+#pragma unroll
+    for (uint32_t j = 0; j < 12; ++j) {
+        const uint32_t v = lane + 32 * j;
+        warpRows[(v / 12) * kRowVectors + v % 12] =
+            accumulate != 0 && v < rows * 12 ? held[v] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    cp_async_wait_all();
     __syncthreads();
+    if (rows == 0) return;
     // The next view's count and first pair are loaded, and its first partials
     // asked into L2, while this view's gradients are computed.
     uint32_t nextCount = live ? touched[sF[0].base + i] : 0u;
@@ -499,11 +567,15 @@ splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t vie
         }
         if (!live || n == 0) continue;
         float gm[3] = {0, 0, 0}, gls[3] = {0, 0, 0}, gq[4] = {0, 0, 0, 0}, glog = 0.0f;
-        view_grads(f, i, means, logScales, quats, logits, sh, g, gm, gls, gq, glog,
-                   [&](int q, float x) { sAcc[q][tid] = __fadd_rn(sAcc[q][tid], x); });
         // The running sums are plain rounded additions (never fused with the
         // product that formed a term), so that they equal the single-view
         // gradients summed in view order.
+        view_grads(f, i, means, logScales, quats, logits, sSh + tid * kShPitch, g, gm, gls, gq, glog,
+                   [&](int q, const float4& x) {
+                       const float4 was = row[q];
+                       row[q] = make_float4(__fadd_rn(was.x, x.x), __fadd_rn(was.y, x.y), __fadd_rn(was.z, x.z),
+                                            __fadd_rn(was.w, x.w));
+                   });
         for (int k = 0; k < 3; ++k) {
             am[k] = __fadd_rn(am[k], gm[k]);
             als[k] = __fadd_rn(als[k], gls[k]);
@@ -511,16 +583,7 @@ splat_backward_views_kernel(const FrameParams* __restrict__ frames, uint32_t vie
         for (int k = 0; k < 4; ++k) aq[k] = __fadd_rn(aq[k], gq[k]);
         alog = __fadd_rn(alog, glog);
     }
-    if (!live) return;
-    for (int k = 0; k < 3; ++k) {
-        gMeans[3 * i + k] = am[k];
-        gLogScales[3 * i + k] = als[k];
-    }
-    for (int k = 0; k < 4; ++k) gQuats[4 * i + k] = aq[k];
-    gLogits[i] = alog;
-#pragma unroll
-    for (int q = 0; q < 12; ++q)
-        shRow[q] = make_float4(sAcc[4 * q][tid], sAcc[4 * q + 1][tid], sAcc[4 * q + 2][tid], sAcc[4 * q + 3][tid]);
+    write_warp(warpRows, rows, first, lane, am, als, aq, alog, gMeans, gLogScales, gQuats, gLogits, gSh);
 }
 
 }  // namespace
