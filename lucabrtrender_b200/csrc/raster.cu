@@ -242,6 +242,10 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     bp.tileShift = 32;
     bp.pairShift = 1;
     uint32_t* emitSlot = nullptr;
+    // A stage's end, for stats that ask for the stages' times. A frame that
+    // does not leaves the events out: each costs a call and, between two
+    // chained kernels, the second's early start.
+    auto mark = [&](int k) { return s->time_stages ? cudaEventRecord(r->ev[k], stream) : cudaSuccess; };
     for (int attempt = 0; attempt < 2; ++attempt) {
         RowFrame rows{};
         if (byRows) {
@@ -286,7 +290,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         uint32_t* bandsOut = byRows ? bands : nullptr;
 
         // --- project, count -------------------------------------------------------
-        LRT_CUDA(r, cudaEventRecord(r->ev[0], stream), "event");
+        LRT_CUDA(r, mark(0), "event");
         uint32_t base = 0, launch = 0;
         uint64_t* depthWords = static_cast<uint64_t*>(r->depthWords.ptr);
         uint64_t* aux = static_cast<uint64_t*>(r->splatAux.ptr);
@@ -330,7 +334,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             base += c.count;
             launch += 1;
         }
-        LRT_CUDA(r, cudaEventRecord(r->ev[1], stream), "event");
+        LRT_CUDA(r, mark(1), "event");
         // --- depth sort of the slots (24-bit keys; ties stay in slot order) ------------
         bool depthInAlt = false;
         LRT_CUDA(r,
@@ -339,7 +343,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                                       depthDigits, true),
                  "depth sort");
         const uint64_t* byDepth = depthInAlt ? static_cast<const uint64_t*>(r->depthWordsAlt.ptr) : depthWords;
-        LRT_CUDA(r, cudaEventRecord(r->ev[4], stream), "event");
+        LRT_CUDA(r, mark(4), "event");
         if (byRows) {
             // --- the splats' runs of tiles, sorted by tile row ------------------------
             rows.sortedWords = byDepth;
@@ -364,7 +368,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             rows.zeroed = static_cast<char*>(r->scanScratch.ptr) + rowsAt;
             rows.scratch = r->rowScratch.ptr;
             LRT_CUDA(r, lrt::launch_row_runs(rows, stream), "runs");
-            LRT_CUDA(r, cudaEventRecord(r->ev[5], stream), "event");
+            LRT_CUDA(r, mark(5), "event");
             // --- every tile's slots in depth order, and its range -----------------------
             LRT_CUDA(r, lrt::launch_row_pairs(rows, stream), "pairs");
             bp.pairShift = 0;
@@ -382,7 +386,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                                              tilePasses != 0 ? tileDigits : nullptr, tilePasses,
                                              static_cast<const uint2*>(r->rowTable.ptr), stream, valueBuf, emitSlot),
                      "emit");
-            LRT_CUDA(r, cudaEventRecord(r->ev[5], stream), "event");
+            LRT_CUDA(r, mark(5), "event");
             // --- stable sort on the tile bits + ranges -------------------------------------------
             bool inAlt = false;
             LRT_CUDA(r,
@@ -406,7 +410,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             LRT_CUDA(r, lrt::launch_tile_order(static_cast<uint2*>(r->ranges.ptr), tiles, tileOrder, tileOrder + tiles,
                                                stream),
                      "tile order");
-        LRT_CUDA(r, cudaEventRecord(r->ev[2], stream), "event");
+        LRT_CUDA(r, mark(2), "event");
 
         // --- blend ------------------------------------------------------------------
         if (train) {
@@ -432,7 +436,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                                        static_cast<float*>(targets->depth), err, stream, tileOrder),
                      "blend");
         }
-        LRT_CUDA(r, cudaEventRecord(r->ev[3], stream), "event");
+        LRT_CUDA(r, mark(3), "event");
         const bool ring = deferred && !train;
         const uint32_t slot = static_cast<uint32_t>(r->ringHead % lrt_rast::kRing);
         LRT_CUDA(r, lrt::launch_publish_counters(counters, ring ? r->ringHostDev + 4 * slot : r->hostCountersDev, stream),
