@@ -733,7 +733,8 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
         const uint32_t excl = incl - mine;
         const float invW = mine != 0 ? 1.0f / static_cast<float>(rw) : 0.0f;
-        const float gate = mine != 0 ? far_edge_gate(ca, cb, cc, cutoff) : INFINITY;
+        const TileTest test = mine != 0 ? tile_test(ca, cb, cc, cutoff) : TileTest{0.0f, 0.0f, -INFINITY, INFINITY};
+        const uint32_t corner = rect.x | (rect.y << 16);   // sides of at most 2^15 tiles
         for (uint32_t c0 = 0; c0 < total; c0 += 32) {
             const uint32_t pos = c0 + lane;
             uint32_t l = 0;
@@ -746,15 +747,22 @@ project_emit_kernel(FrameParams fArg, const FrameParams* __restrict__ fDev, Src 
             const uint32_t k = pos - __shfl_sync(0xFFFFFFFFu, excl, src);
             const uint32_t oW = __shfl_sync(0xFFFFFFFFu, rw, src);
             const float oInv = __shfl_sync(0xFFFFFFFFu, invW, src);
-            const uint32_t oX = __shfl_sync(0xFFFFFFFFu, rect.x, src), oY = __shfl_sync(0xFFFFFFFFu, rect.y, src);
+            const uint32_t oCorner = __shfl_sync(0xFFFFFFFFu, corner, src);
             const float ocx = __shfl_sync(0xFFFFFFFFu, cx, src), ocy = __shfl_sync(0xFFFFFFFFu, cy, src);
             const float oa = __shfl_sync(0xFFFFFFFFu, ca, src), ob = __shfl_sync(0xFFFFFFFFu, cb, src);
-            const float oc = __shfl_sync(0xFFFFFFFFu, cc, src), ocut = __shfl_sync(0xFFFFFFFFu, cutoff, src);
-            const float ogate = __shfl_sync(0xFFFFFFFFu, gate, src);
+            const float oc = __shfl_sync(0xFFFFFFFFu, cc, src);
+            const TileTest otest{__shfl_sync(0xFFFFFFFFu, test.slopeX, src), __shfl_sync(0xFFFFFFFFu, test.slopeY, src),
+                                 __shfl_sync(0xFFFFFFFFu, test.sure, src), __shfl_sync(0xFFFFFFFFu, test.gate, src)};
             uint32_t dx = 0, dy = 0;
             mask_bit_tile(k, oW, oInv, dx, dy);
-            const bool hit = pos < total && tile_touched(f.width, f.height, ocx, ocy, oa, ob, oc, ocut, oX + dx, oY + dy,
-                                                         ogate);
+            const uint32_t tx = (oCorner & 0xFFFFu) + dx, ty = (oCorner >> 16) + dy;
+            const Touch touch = pos < total ? tile_touch(f.width, f.height, ocx, ocy, oa, ob, oc, otest, tx, ty) : Touch::kNo;
+            bool hit = touch == Touch::kYes;
+            if (__any_sync(0xFFFFFFFFu, touch == Touch::kUnsure)) {
+                const float ocut = __shfl_sync(0xFFFFFFFFu, cutoff, src);
+                if (touch == Touch::kUnsure)
+                    hit = tile_touched(f.width, f.height, ocx, ocy, oa, ob, oc, ocut, tx, ty, otest.gate);
+            }
             const uint32_t bal = __ballot_sync(0xFFFFFFFFu, hit);
             if (mine != 0) {
                 const uint32_t lo = max(excl, c0), hi = min(incl, c0 + 32);
