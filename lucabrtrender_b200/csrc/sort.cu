@@ -15,10 +15,10 @@
 //      keys are warp-striped, so a warp's item j covers 32 consecutive keys
 //      and items are visited in order), and across warps with per-warp
 //      digit counts,
-//   3. publishes its per-digit counts and resolves the prefix of all earlier
+//   3. publishes its per-digit counts, scatters its keys (and values) into
+//      shared memory in digit order, and resolves the prefix of all earlier
 //      partitions by decoupled look-back (bounded waits),
-//   4. scatters keys (and values) into shared memory in digit order, then
-//      writes them out so that consecutive threads write consecutive slots.
+//   4. writes the keys out so that consecutive threads write consecutive slots.
 // Only the key bits asked for are sorted: the pass count is ceil(bits / 8).
 // Key types: uint32 and uint64, with or without uint32 values. The key count
 // is read on the device (at most `cap`), or is `cap` when no count is given.
@@ -60,7 +60,14 @@ constexpr uint32_t kSmallSortMax = (1u << 30) - 1;   // the most keys 32-bit wor
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr uint32_t kMaxPasses = 8;
 constexpr uint32_t kHistThreads = 512;
-constexpr uint32_t kLookWords = 4;   // earlier partitions' status words a look-back step reads
+// Earlier partitions' status words a look-back step reads. Partitions of one
+// wave publish at once, so a step's words set how fast the chain of prefixes
+// runs down the wave; more words read more partitions twice. The five passes
+// of 12 views' 1M splats, and of a frame of 500k slots at 1366x768: 1.026 and
+// 0.0708 ms with four words a step and the keys scattered after the look-back;
+// with the keys scattered before it 0.956 and 0.0664 at eight words, 1.049 and
+// 0.0729 at sixteen, 1.211 and 0.0838 at thirty-two.
+constexpr uint32_t kLookWords = 8;
 
 // 256-wide exclusive scan across the block (one value per thread).
 __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_t* sWarp) {
@@ -208,6 +215,19 @@ onesweep_kernel(const K* __restrict__ kin, K* __restrict__ kout, const uint32_t*
     const uint32_t blockStart = block_exclusive_scan_256(count, sScan);
     const uint32_t globalStart = block_exclusive_scan_256(hist[tid], sScan);
     sBlockStart[tid] = blockStart;
+    sGlobal[tid] = globalStart - blockStart;
+    __syncthreads();
+
+    // Scatter into shared memory in digit order: before the look-back, so
+    // that the keys leave their registers to its words, and the earlier
+    // partitions have this long to publish.
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j) {
+        const uint32_t d = dig[j];
+        const uint32_t at = sBlockStart[d] + sWarpHist[warp][d] + rank[j];
+        sKeys[at] = key[j];
+        if (kValues) sVals[at] = val[j];
+    }
 
     // The look-back reads kLookWords earlier partitions' words at once (their
     // loads in flight together) and sums them in order up to the first one
@@ -248,17 +268,7 @@ onesweep_kernel(const K* __restrict__ kin, K* __restrict__ kout, const uint32_t*
         }
         mine.store(kFlagInclusive | static_cast<W>(prefix + count), cuda::memory_order_relaxed);
     }
-    sGlobal[tid] = globalStart + prefix - blockStart;
-    __syncthreads();
-
-    // Scatter into shared memory in digit order.
-#pragma unroll
-    for (uint32_t j = 0; j < kItems; ++j) {
-        const uint32_t d = dig[j];
-        const uint32_t at = sBlockStart[d] + sWarpHist[warp][d] + rank[j];
-        sKeys[at] = key[j];
-        if (kValues) sVals[at] = val[j];
-    }
+    sGlobal[tid] += prefix;
     __syncthreads();
 
     // Write out: slot i of the block goes to sGlobal[digit] + i.
