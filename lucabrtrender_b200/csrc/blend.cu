@@ -531,12 +531,13 @@ __global__ void __launch_bounds__(kBlendThreads / kBlendPix)
 blend_composite_kernel(BlendParams bp, const uint2* __restrict__ ranges, const unsigned long long* __restrict__ pairs,
                        const ProjRecord* __restrict__ proj, float4* __restrict__ colourOut,
                        float* __restrict__ depthOut, const float4* __restrict__ underColour,
-                       const float* __restrict__ underDepth, uint32_t* __restrict__ err) {
+                       const float* __restrict__ underDepth, uint32_t* __restrict__ err,
+                       const uint32_t* __restrict__ order) {
     __shared__ BlendShared sh;
     __shared__ CompositeShared comp;
     blend_init(sh);
     uint32_t phase = 0;
-    const uint32_t tile = blockIdx.x;
+    const uint32_t tile = order != nullptr ? order[blockIdx.x] : blockIdx.x;
     blend_tile<false, kWords, true>(bp, tile, tile % bp.tilesX, tile / bp.tilesX, ranges, pairs, nullptr, proj, colourOut,
                             depthOut, nullptr, nullptr, err, sh, phase, underColour, underDepth, &comp);
 }
@@ -765,13 +766,13 @@ cudaError_t launch_blend(const BlendParams& bp, const uint2* ranges, const uint6
 
 cudaError_t launch_blend_composite(const BlendParams& bp, const uint2* ranges, const uint64_t* pairs,
                                   const ProjRecord* proj, float4* colour, float* depth, const float4* underColour,
-                                  const float* underDepth, uint32_t* err, cudaStream_t stream) {
+                                  const float* underDepth, uint32_t* err, cudaStream_t stream, const uint32_t* order) {
     const uint32_t tiles = bp.tilesX * bp.tilesY;
     if (tiles == 0) return cudaSuccess;
     const auto kernel = bp.pairShift != 0 ? blend_composite_kernel<true> : blend_composite_kernel<false>;
     kernel<<<tiles, kBlendThreads / kBlendPix, 0, stream>>>(
         bp, ranges, reinterpret_cast<const unsigned long long*>(pairs), proj, colour, depth, underColour, underDepth,
-        err);
+        err, order);
     return cudaGetLastError();
 }
 

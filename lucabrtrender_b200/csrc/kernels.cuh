@@ -174,6 +174,12 @@ cudaError_t launch_publish_counters(const uint32_t* counters, uint32_t* hostMapp
 // The frame's tiles busiest first (by buckets of log2 of their pair counts),
 // the order the blends below launch them in when given one; scratch holds
 // tile_order_scratch_bytes(tiles).
+// Frames of fewer tiles than kOrderMinTiles start all their blocks at once and
+// gain nothing from an order: 192 tiles (3k splats, 250x190) blend 17.0 us in
+// index order and 17.3 busiest first, 294 tiles (a 20k-splat training frame)
+// 57.4 and 56.9, for 3.6 us of ordering (9.8 with the backward's). At 1024
+// tiles (100k, 512x512) an SM's share still matters: 63.6 and 55.8.
+constexpr uint32_t kOrderMinTiles = 512;
 size_t tile_order_scratch_bytes(uint32_t tiles);
 cudaError_t launch_tile_order(const uint2* ranges, uint32_t tiles, uint32_t* order, uint32_t* scratch,
                               cudaStream_t stream, const uint32_t* work = nullptr);
@@ -193,7 +199,7 @@ cudaError_t launch_blend(const BlendParams& bp, const uint2* ranges, const uint6
 // layer (underColour may be null: discs only).
 cudaError_t launch_blend_composite(const BlendParams& bp, const uint2* ranges, const uint64_t* pairs,
                                   const ProjRecord* proj, float4* colour, float* depth, const float4* underColour,
-                                  const float* underDepth, uint32_t* err, cudaStream_t stream);
+                                  const float* underDepth, uint32_t* err, cudaStream_t stream, const uint32_t* order);
 cudaError_t launch_blend_batch(const BlendParams& bp, const ViewParams* views, uint32_t viewCount, const uint2* ranges,
                                const uint64_t* pairs, const ProjRecord* proj, uint32_t totalTiles, uint32_t* queue,
                                uint32_t* err, uint32_t blocks, cudaStream_t stream);

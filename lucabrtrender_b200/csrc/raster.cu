@@ -403,12 +403,11 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                      "ranges");
             r->debugLow = nullptr;
         }
-        // The blend takes the tiles busiest first (the composite blend keeps
-        // index order).
-        uint32_t* tileOrder = composite ? nullptr : static_cast<uint32_t*>(r->tileOrder.ptr);
+        // The blend takes the tiles busiest first, where they outnumber the
+        // blocks that start at once.
+        uint32_t* tileOrder = tiles >= lrt::kOrderMinTiles ? static_cast<uint32_t*>(r->tileOrder.ptr) : nullptr;
         if (tileOrder != nullptr)
-            LRT_CUDA(r, lrt::launch_tile_order(static_cast<uint2*>(r->ranges.ptr), tiles, tileOrder, tileOrder + tiles,
-                                               stream),
+            LRT_CUDA(r, lrt::launch_tile_order(static_cast<uint2*>(r->ranges.ptr), tiles, tileOrder, tileOrder + tiles, stream),
                      "tile order");
         LRT_CUDA(r, mark(2), "event");
 
@@ -427,7 +426,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                          bp, static_cast<uint2*>(r->ranges.ptr), sorted, static_cast<ProjRecord*>(r->proj.ptr),
                          static_cast<float4*>(targets->colour), static_cast<float*>(targets->depth),
                          under != nullptr ? static_cast<const float4*>(under->colour) : nullptr,
-                         under != nullptr ? static_cast<const float*>(under->depth) : nullptr, err, stream),
+                         under != nullptr ? static_cast<const float*>(under->depth) : nullptr, err, stream, tileOrder),
                      "blend");
         } else {
             LRT_CUDA(r,
@@ -1060,13 +1059,15 @@ int lrt_rast_train_backward(lrt_rast* r, const void* gradColour, lrt_train_grads
     const BlendParams& tb = r->trainBlend;
     const uint32_t bTiles = tb.tilesX * tb.tilesY;
     const lrt::ChainScope chain(uint64_t{tb.width} * tb.height >= lrt::kChainMinPixels);
-    uint32_t* bOrder = static_cast<uint32_t*>(r->tileOrder.ptr);
-    uint32_t* bScratch = bOrder + bTiles;
-    uint32_t* bWork = bScratch + lrt::tile_order_scratch_bytes(bTiles) / 4;
-    LRT_CUDA(r,
-             lrt::launch_tile_backward_order(static_cast<uint2*>(r->ranges.ptr), static_cast<uint32_t*>(r->pixLast.ptr),
-                                             tb.width, tb.height, tb.tilesX, bTiles, bOrder, bScratch, bWork, stream),
-             "backward tile order");
+    uint32_t* bOrder = bTiles >= lrt::kOrderMinTiles ? static_cast<uint32_t*>(r->tileOrder.ptr) : nullptr;
+    if (bOrder != nullptr) {
+        uint32_t* bScratch = bOrder + bTiles;
+        uint32_t* bWork = bScratch + lrt::tile_order_scratch_bytes(bTiles) / 4;
+        LRT_CUDA(r,
+                 lrt::launch_tile_backward_order(static_cast<uint2*>(r->ranges.ptr), static_cast<uint32_t*>(r->pixLast.ptr),
+                                                 tb.width, tb.height, tb.tilesX, bTiles, bOrder, bScratch, bWork, stream),
+                 "backward tile order");
+    }
     LRT_CUDA(r,
              lrt::launch_blend_backward(r->trainBlend, static_cast<uint2*>(r->ranges.ptr), r->trainSorted,
                                         r->trainSortedValues, r->trainEmitSlot, static_cast<ProjRecord*>(r->proj.ptr),
