@@ -1043,7 +1043,9 @@ int lrt_rast_train_backward(lrt_rast* r, const void* gradColour, lrt_train_grads
     cudaStream_t stream = static_cast<cudaStream_t>(streamPtr);
     // A forward that ran without waiting has not reported its pair count yet:
     // the backward is enqueued over the pair buffer's capacity (every read
-    // stays inside the buffers), and the forward's counts are read once the
+    // and write stays inside the buffers: a frame that overflowed keeps only
+    // pairs whose emit indices lie below the capacity it ran with, or, made
+    // from runs, no pairs), and the forward's counts are read once the
     // backward is queued behind it, so the device never waits for the host
     // here. If that frame overflowed, the call returns OVERFLOW and the
     // gradients it wrote are not to be used.

@@ -276,8 +276,14 @@ __device__ __forceinline__ uint32_t strided_lookback(unsigned long long* word, s
 }
 
 // Whether the frame's runs are whole: they fit, and no earlier wait gave up.
+// A training frame's pairs have to fit as well: cut at the buffer's end in
+// tile order, the ones left would hold emit indices up to the frame's total,
+// and the backward, which may be enqueued before the counts are read, writes
+// a pair's partials at its emit index. Such a frame gets no pairs (its ranges
+// stay empty) and is reported as overflowed.
 __device__ __forceinline__ bool runs_whole(const RowFrame& f, uint32_t n) {
-    return n != 0 && n <= f.runCap && (f.counters[2] & (kErrTimeout | kErrTooManyPairs)) == 0;
+    return n != 0 && n <= f.runCap && (f.counters[2] & (kErrTimeout | kErrTooManyPairs)) == 0 &&
+           (f.pairEmit == nullptr || f.counters[1] <= f.pairCap);
 }
 
 // Bound by latency (each run gathers its splat's mask and rectangle from L2)

@@ -12,6 +12,7 @@ import pytest
 import torch
 
 import lucabrtrender_b200 as L
+from lucabrtrender_b200 import _abi
 import helpers as H
 import oracle as ora
 import train_fixtures as TF
@@ -104,3 +105,35 @@ def test_enqueued_frames_that_outgrow_their_buffers():
         assert np.array_equal(targets.colour.cpu().numpy().view(np.uint32), want["colour"].view(np.uint32))
     finally:
         r.close()
+
+
+def test_an_enqueued_training_step_that_outgrows_its_buffer():
+    """The step's backward is enqueued over the frame before its counts are
+    read: it reports OVERFLOW, and the step run again has the image and the
+    gradients of a handle that never overflowed, bit for bit. (A frame cut at
+    the buffer's end in tile order would hold emit indices past it.)"""
+    n, width, height = 30000, 800, 640
+    p = TF.make_params(n, 3, log_scale_mean=-1.7, log_scale_sigma=0.8)
+    far, settings = TF.frame(width, height, eye=(0.0, 0.0, 6.0))    # 2.6M pairs
+    near, _ = TF.frame(width, height, eye=(0.0, 0.0, 3.0))          # 8.2M
+    target = torch.rand(height, width, 3, generator=torch.Generator().manual_seed(2)).cuda()
+
+    def step(r, cam):
+        t = {k: torch.from_numpy(v).cuda().requires_grad_(True) for k, v in p.items()}
+        colour, _ = L.rasterize(t["means"], t["log_scales"], t["quats"], t["logits"], t["sh"], cam, settings, r)
+        L.l1_loss(colour, target, r).backward()
+        return [colour.detach()] + [v.grad for v in t.values()]
+
+    r, fresh = L.TileRasterizer.create(0), L.TileRasterizer.create(0)
+    try:
+        for _ in range(3):   # the first sizes the buffers, the second leaves a quarter free, the third is enqueued
+            step(r, far)
+        assert r.debug_arrays()["pairs"].numel() >= max(MIN_PAIRS, MIN_PER_SPLAT * n)
+        with pytest.raises(L.LrtError) as info:
+            step(r, near)
+        assert info.value.code == _abi.OVERFLOW
+        for a, b in zip(step(r, near), step(fresh, near)):
+            assert torch.equal(a, b)
+    finally:
+        r.close()
+        fresh.close()
