@@ -205,7 +205,8 @@ typedef struct lrt_debug_view {
     const void* pairs;           /* uint64 per pair, sorted: tile | depth key | slot (see pair_*) */
     const void* ranges;          /* uint32 x2 per tile: [start, end) into pairs */
     uint32_t slots, pairs_count, tiles, slot_bits;
-    uint32_t depth_bits, tile_bits, visible, reserved;
+    uint32_t depth_bits, tile_bits, visible;
+    uint32_t from_runs;          /* 1: the frame's pairs were made from the splats' runs of tiles, 0: from sorted words */
 } lrt_debug_view;
 
 typedef struct lrt_rast lrt_rast;
@@ -262,8 +263,9 @@ int lrt_rast_render_async(lrt_rast* rast, const lrt_projection* projection,
                           const lrt_render_settings* settings, lrt_targets* targets, void* stream);
 
 /* Waits for every enqueued frame. Returns LRT_OVERFLOW when any of them
- * emitted more pairs than the buffer held (their images are incomplete; the
- * buffers are grown, so drawing them again succeeds), LRT_TIMEOUT when a
+ * emitted more pairs, or more runs of tiles, than the buffers held (their
+ * images are incomplete; the buffers are grown or the next frame's form is
+ * chosen to fit, so drawing them again succeeds), LRT_TIMEOUT when a
  * bounded device wait gave up, else LRT_OK. `stats` (may be NULL) receives
  * the splats, visible splats and pairs of the last frame. */
 int lrt_rast_settle(lrt_rast* rast, lrt_frame_stats* stats);
@@ -357,7 +359,7 @@ typedef struct lrt_train_grads {
  * queued behind it, and the stats then carry only the splat count. Such a
  * frame's counts and status are checked by lrt_rast_train_backward, which
  * returns LRT_OVERFLOW (buffers grown; run the step again) if the frame
- * emitted more pairs than the buffers held. */
+ * emitted more pairs, or more runs of tiles, than the buffers held. */
 int lrt_rast_train_forward(lrt_rast* rast, const lrt_projection* projection, const lrt_train_params* params,
                            const lrt_render_settings* settings, lrt_targets* targets, lrt_frame_stats* stats,
                            void* stream);

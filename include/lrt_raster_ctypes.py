@@ -157,7 +157,7 @@ class DebugView(C.Structure):
         ("proj", C.c_void_p), ("rects", C.c_void_p), ("touched", C.c_void_p), ("depth_keys", C.c_void_p),
         ("pairs", C.c_void_p), ("ranges", C.c_void_p),
         ("slots", C.c_uint32), ("pairs_count", C.c_uint32), ("tiles", C.c_uint32), ("slot_bits", C.c_uint32),
-        ("depth_bits", C.c_uint32), ("tile_bits", C.c_uint32), ("visible", C.c_uint32), ("reserved", C.c_uint32),
+        ("depth_bits", C.c_uint32), ("tile_bits", C.c_uint32), ("visible", C.c_uint32), ("from_runs", C.c_uint32),
     ]
 
 

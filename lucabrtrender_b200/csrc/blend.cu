@@ -595,15 +595,25 @@ cudaError_t launch_ranges(const uint64_t* pairs, const uint32_t* dCount, uint32_
 
 namespace {
 template <bool kChained>
-__global__ void publish_counters_kernel(const uint32_t* __restrict__ counters, uint32_t* hostMapped) {
+__global__ void publish_counters_kernel(const uint32_t* __restrict__ counters, const uint32_t* __restrict__ bands,
+                                        uint32_t* hostMapped) {
     chained_entry<kChained>();
     if (threadIdx.x < 4) hostMapped[threadIdx.x] = counters[threadIdx.x];
+    unsigned long long runs = 0;
+    if (bands != nullptr) {
+        for (uint32_t k = threadIdx.x; k < kMaxBands; k += 32) runs += bands[k];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) runs += __shfl_xor_sync(0xFFFFFFFFu, runs, d);
+    }
+    if (threadIdx.x == 0) hostMapped[4] = static_cast<uint32_t>(min(runs, 0xFFFFFFFFull));
     __threadfence_system();
 }
 }  // namespace
 
-cudaError_t launch_publish_counters(const uint32_t* counters, uint32_t* hostMapped, cudaStream_t stream) {
-    return launch_chained(publish_counters_kernel<true>, publish_counters_kernel<false>, dim3(1), dim3(32), 0, stream, counters, hostMapped);
+cudaError_t launch_publish_counters(const uint32_t* counters, const uint32_t* bands, uint32_t* hostMapped,
+                                    cudaStream_t stream) {
+    return launch_chained(publish_counters_kernel<true>, publish_counters_kernel<false>, dim3(1), dim3(32), 0, stream,
+                          counters, bands, hostMapped);
 }
 
 namespace {

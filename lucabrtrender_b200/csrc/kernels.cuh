@@ -164,12 +164,14 @@ struct ZeroRegion {
 constexpr uint32_t kZeroRegions = 6;
 cudaError_t launch_zero_regions(const ZeroRegion* regions, uint32_t count, cudaStream_t stream);
 
-// The frame's four counters stored into pinned host memory by a kernel
+// The frame's four counters, and with `bands` (may be null) the runs they add
+// up to as a fifth word, else zero, stored into pinned host memory by a kernel
 // (`hostMapped` is the device's address of that memory), not by a copy: a
 // device-to-host copy queues behind whatever the copy engine already holds,
 // such as a caller's readback of the previous image, and the frame's stream
 // would wait for it.
-cudaError_t launch_publish_counters(const uint32_t* counters, uint32_t* hostMapped, cudaStream_t stream);
+cudaError_t launch_publish_counters(const uint32_t* counters, const uint32_t* bands, uint32_t* hostMapped,
+                                    cudaStream_t stream);
 
 // The frame's tiles busiest first (by buckets of log2 of their pair counts),
 // the order the blends below launch them in when given one; scratch holds

@@ -200,12 +200,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // aggregates up to it are summed across the warp. A partition in the window
 // that has published nothing yet makes the warp read the window again
 // (bounded: after kSpinLimit polls kErrTimeout is raised and the walk
-// ends). The frame's last partition writes the pair total to counters[1].
+// ends). The frame's last partition writes the total to counters[1], and
+// raises `tooMany` where that has no room for it.
 // Called by warp 0 only; lane 0's result is the block's base.
 __device__ __forceinline__ unsigned long long frame_lookback(uint64_t* __restrict__ status, uint32_t g,
                                                              uint32_t lastPartition, uint32_t blockTotal,
                                                              uint32_t* __restrict__ counters,
-                                                             uint32_t* __restrict__ err) {
+                                                             uint32_t* __restrict__ err,
+                                                             uint32_t tooMany = kErrTooManyPairs) {
     const uint32_t lane = threadIdx.x & 31u;
     uint64_t prefix = 0;
     if (lane == 0) {
@@ -248,7 +250,7 @@ __device__ __forceinline__ unsigned long long frame_lookback(uint64_t* __restric
     }
     if (lane == 0 && g == lastPartition) {
         const uint64_t all = prefix + blockTotal;
-        if (all > 0xFFFFFFFFull) atomicOr(err, kErrTooManyPairs);
+        if (all > 0xFFFFFFFFull) atomicOr(err, tooMany);
         counters[1] = static_cast<uint32_t>(all);
     }
     return prefix;

@@ -34,7 +34,7 @@ struct lrt_rast {
     DeviceBuffer ranges;                                 // per tile
     DeviceBuffer tileOrder;                              // per tile: the blend's launch order
     DeviceBuffer scanScratch, sortScratch;               // look-back status words, tickets
-    DeviceBuffer counters;                               // visible, pairs, err, algo err
+    DeviceBuffer counters;                               // visible, pairs, err, row table entries or algo err, runs
     DeviceBuffer algoKeysAlt, algoValsAlt;               // lrt_radix_sort's ping-pong buffers
     DeviceBuffer depthWords, depthWordsAlt, splatAux;    // per slot: depth words (two-step frames), aux words
     DeviceBuffer rowTable;                               // large splats' rows (first column, count)
@@ -50,7 +50,9 @@ struct lrt_rast {
     // counts copied to the host; ev[7..9]: the training backward's times.
     cudaEvent_t ev[10] = {};
     uint32_t splatCap = 0, pairCap = 0, tileCap = 0;
-    uint32_t seenPairs = 0, seenSlots = 0;   // the last single frame whose counts were read: its pairs and splats
+    // The last single frame whose counts were read: its pairs, its splats and
+    // its runs of tiles (0 where they were not counted).
+    uint32_t seenPairs = 0, seenSlots = 0, seenRuns = 0;
     lrt_debug_view debug{};
     // Training: what the backward pass needs from its forward.
     DeviceBuffer pairValues, pairValuesAlt, pairOffsets, pixState, pixLast, partials;
@@ -79,8 +81,8 @@ struct lrt_rast {
     bool backwardTimed = false;   // ev[7..9] hold a training backward's times
     // Plain frames enqueued by lrt_rast_render_async: their counts land in a
     // ring of pinned slots, each with the event that marks its frame done.
-    static constexpr uint32_t kRing = 16;
-    uint32_t* ringHost = nullptr;               // pinned, 4 words per slot
+    static constexpr uint32_t kRing = 16, kRingWords = 8;
+    uint32_t* ringHost = nullptr;               // pinned, kRingWords per slot
     uint32_t* ringHostDev = nullptr;            // the device's address of ringHost
     cudaEvent_t ringEvent[kRing] = {};
     uint32_t ringCap[kRing] = {};               // the pair capacity each frame ran with
@@ -163,6 +165,14 @@ inline uint32_t grow(uint32_t have, uint32_t need) {
     uint64_t size = std::max<uint32_t>(have, 1024);
     while (size < need) size = size * 3 / 2;
     return static_cast<uint32_t>(std::min<uint64_t>(size, 0xFFFFFFFFull));
+}
+
+// A single frame's published counters (launch_publish_counters), kept for the
+// next frame's choice of form.
+inline void note_counts(lrt_rast* r, const uint32_t* counts, uint32_t slots) {
+    r->seenPairs = counts[1];
+    r->seenSlots = slots;
+    r->seenRuns = counts[4];
 }
 
 inline cudaError_t ensure(DeviceBuffer& b, size_t bytes) {

@@ -9,7 +9,8 @@
 // The reference reads the counts back in the middle of the frame to size the
 // pair buffers; here the pairs go into a buffer sized before the frame, and a
 // frame that reports more pairs than it held is drawn again with room for
-// them (once per growth, so steady frames never repeat).
+// them (once per growth, and once more where its runs of tiles turn out to be
+// more than its pairs, so steady frames never repeat).
 //
 // Buffers belong to the handle and grow by 1.5x (TileRasterizer.cpp:26-32);
 // targets and clouds belong to the caller. Stage times come from CUDA events
@@ -41,7 +42,7 @@ int lrt_rast_create(lrt_rast** out, int device) {
     lrt_rast* r = new lrt_rast();
     r->device = device;
     bool ok = cudaMallocHost(reinterpret_cast<void**>(&r->hostCounters), 64) == cudaSuccess &&
-              cudaMallocHost(reinterpret_cast<void**>(&r->ringHost), lrt_rast::kRing * 16) == cudaSuccess &&
+              cudaMallocHost(reinterpret_cast<void**>(&r->ringHost), lrt_rast::kRing * lrt_rast::kRingWords * 4) == cudaSuccess &&
               cudaHostGetDevicePointer(reinterpret_cast<void**>(&r->hostCountersDev), r->hostCounters, 0) ==
                   cudaSuccess &&
               cudaHostGetDevicePointer(reinterpret_cast<void**>(&r->ringHostDev), r->ringHost, 0) == cudaSuccess &&
@@ -159,12 +160,20 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     // 0.211 / 0.180 (300k, 1366x768); 13.6 and 1.3M 0.122 / 0.119, 7 and 0.7M
     // 0.092 / 0.103 (100k, 512x512); 160 and 156M 3.69 / 1.83 (1M, 4K). The
     // counts are those of the last frame of as many splats that was read.
+    // A splat has at most a run a tile row where each of its rows is one run,
+    // and one a tile of its rectangle where one is not (long thin splats seen
+    // at a slant: up to eight times the pairs in a frame of those). Frames
+    // with more runs than pairs take words. A frame that waits may learn its
+    // runs by not holding them, and is then drawn again; one that does not
+    // wait takes words, and counts its runs, until they are known.
     constexpr uint32_t kRunsMinPairs = 1u << 21, kRunsMinPerSplat = 6;
     const bool rowsAllowed = tilesX <= lrt::kMaxBands && tilesY <= lrt::kMaxBands;
-    auto runs_pay = [&](uint32_t pairCount) {
-        return rowsAllowed && pairCount >= kRunsMinPairs && pairCount / kRunsMinPerSplat >= slots;
+    bool countRuns = false, byRows = false;
+    auto choose_form = [&](uint32_t pairCount, uint32_t runCount, bool waits) {
+        countRuns = rowsAllowed && pairCount >= kRunsMinPairs && pairCount / kRunsMinPerSplat >= slots;
+        byRows = countRuns && (runCount != 0 ? runCount <= pairCount : waits);
     };
-    bool byRows = r->seenSlots == slots && runs_pay(r->seenPairs);
+    if (r->seenSlots == slots) choose_form(r->seenPairs, r->seenRuns, !deferred);
 
     // Buffers (TileRasterizer.cpp:105-177).
     if (slots > r->splatCap) {
@@ -204,7 +213,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         r->tileCap = tiles;
     }
     // Pairs are emitted on the device into a buffer of the capacity known
-    // before the frame; a frame that emits more is drawn again once, with the
+    // before the frame; a frame that emits more is drawn again, with the
     // buffers grown to the count it reported.
     if (r->pairCap == 0)
         r->pairCap = std::max<uint32_t>(1024, static_cast<uint32_t>(std::min<uint64_t>(uint64_t{slots} * 4, 0xFFFFFFFFull)));
@@ -246,15 +255,18 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     // does not leaves the events out: each costs a call and, between two
     // chained kernels, the second's early start.
     auto mark = [&](int k) { return s->time_stages ? cudaEventRecord(r->ev[k], stream) : cudaSuccess; };
-    for (int attempt = 0; attempt < 2; ++attempt) {
+    // Three attempts at most: one whose pairs do not fit; one with room for
+    // them, as runs not counted before; and, should those be more than the
+    // pairs, one as words, with room for every pair.
+    constexpr int kAttempts = 3;
+    for (int attempt = 0; attempt < kAttempts; ++attempt) {
         RowFrame rows{};
+        if (countRuns) LRT_CUDA(r, ensure(r->runCounts, size_t{r->splatCap} * sizeof(uint2)), "run counts");
         if (byRows) {
-            // A splat has a run where it has pairs, but for the empty rows at
-            // the ends of a few large ones' rectangles.
+            // Room for a run a pair, and a quarter more.
             rows.runCap = static_cast<uint32_t>(
                 std::min<uint64_t>(uint64_t{r->pairCap} + r->pairCap / 4 + 1024, 0xFFFFF000ull));
             rows.pairCap = r->pairCap;
-            LRT_CUDA(r, ensure(r->runCounts, size_t{r->splatCap} * sizeof(uint2)), "run counts");
             LRT_CUDA(r, ensure(r->runs, size_t{rows.runCap} * 8), "runs");
             LRT_CUDA(r, ensure(r->pairSlots, size_t{r->pairCap} * 4), "pairs");
             LRT_CUDA(r, ensure(r->rowScratch, lrt::row_scratch_bytes(slots, rows.runCap, tilesX)), "row scratch");
@@ -286,8 +298,8 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         uint64_t* pairBuf = static_cast<uint64_t*>(r->pairs.ptr);
         uint32_t* valueBuf = train && !lowIsEmit && !byRows ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
         emitSlot = train && lowIsEmit && !byRows ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
-        uint2* runCounts = byRows ? static_cast<uint2*>(r->runCounts.ptr) : nullptr;
-        uint32_t* bandsOut = byRows ? bands : nullptr;
+        uint2* runCounts = countRuns ? static_cast<uint2*>(r->runCounts.ptr) : nullptr;
+        uint32_t* bandsOut = countRuns ? bands : nullptr;
 
         // --- project, count -------------------------------------------------------
         LRT_CUDA(r, mark(0), "event");
@@ -438,7 +450,9 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         LRT_CUDA(r, mark(3), "event");
         const bool ring = deferred && !train;
         const uint32_t slot = static_cast<uint32_t>(r->ringHead % lrt_rast::kRing);
-        LRT_CUDA(r, lrt::launch_publish_counters(counters, ring ? r->ringHostDev + 4 * slot : r->hostCountersDev, stream),
+        LRT_CUDA(r,
+                 lrt::launch_publish_counters(
+                     counters, bandsOut, ring ? r->ringHostDev + lrt_rast::kRingWords * slot : r->hostCountersDev, stream),
                  "readback");
         LRT_CUDA(r, cudaEventRecord(r->frameDone, stream), "event");
         r->frameDoneSet = true;
@@ -460,6 +474,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             r->debug.slot_bits = 32u;
             r->debug.depth_bits = 0u;
             r->debug.tile_bits = tileBits;
+            r->debug.from_runs = byRows ? 1u : 0u;
             r->pendingStream = stream;
             if (train) LRT_CUDA(r, cudaEventRecord(r->ev[6], stream), "event");
             if (train) {
@@ -484,14 +499,12 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         visible = r->hostCounters[0];
         pairs = r->hostCounters[1];
         statusBits = r->hostCounters[2];
-        r->seenPairs = pairs;
-        r->seenSlots = slots;
+        note_counts(r, r->hostCounters, slots);
         if (statusBits & lrt::kErrTooManyPairs) return fail(r, LRT_UNSUPPORTED, "more than 2^32 pairs in one frame");
-        if (pairs <= r->pairCap && (statusBits & lrt::kErrOverflow) == 0) break;
-        // Draw again with room for every pair (and every run).
-        r->pairCap = grow(r->pairCap, std::max(pairs, r->pairCap + 1));
-        byRows = runs_pay(pairs);
-        statusBits &= ~lrt::kErrOverflow;
+        if ((pairs <= r->pairCap && (statusBits & lrt::kErrRuns) == 0) || attempt + 1 == kAttempts) break;
+        // Draw again with room for every pair.
+        r->pairCap = grow(r->pairCap, pairs);
+        choose_form(pairs, r->seenRuns, true);
     }
     // Rows the frame's large splats asked for beyond the row table: the next
     // frame's table holds them (this one planned those rows again).
@@ -509,6 +522,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     r->debug.slot_bits = 32u;
     r->debug.depth_bits = 0u;
     r->debug.tile_bits = tileBits;
+    r->debug.from_runs = byRows ? 1u : 0u;
     r->debug.visible = visible;
     r->trainReady = false;
     r->trainPending = false;
@@ -538,7 +552,8 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - frameStart).count();
     }
     if (statusBits & lrt::kErrTimeout) return fail(r, LRT_TIMEOUT, "a bounded device wait gave up");
-    if (statusBits & lrt::kErrOverflow || pairs > r->pairCap) return fail(r, LRT_OVERFLOW, "pair capacity exceeded");
+    if ((statusBits & (lrt::kErrOverflow | lrt::kErrRuns)) != 0 || pairs > r->pairCap)
+        return fail(r, LRT_OVERFLOW, "pair capacity exceeded");
     return LRT_OK;
 }
 
@@ -585,15 +600,14 @@ bool read_oldest(lrt_rast* r, bool wait) {
         cudaGetLastError();   // cudaErrorNotReady is not an error to keep
         return false;
     }
-    const uint32_t* c = r->ringHost + 4 * slot;
+    const uint32_t* c = r->ringHost + lrt_rast::kRingWords * slot;
     r->asyncVisible = c[0];
     r->asyncPairs = c[1];
     r->plainSeenPairs = c[1];
-    r->seenPairs = c[1];
-    r->seenSlots = r->ringSlots[slot];
-    if (c[1] > r->ringCap[slot] || (c[2] & (lrt::kErrTooManyPairs | lrt::kErrOverflow)) != 0) {
+    note_counts(r, c, r->ringSlots[slot]);
+    if (c[1] > r->ringCap[slot] || (c[2] & (lrt::kErrTooManyPairs | lrt::kErrRuns)) != 0) {
         r->asyncOverflows += 1;
-        r->pairCap = std::max(r->pairCap, grow(r->pairCap, std::max(c[1], r->ringCap[slot] + 1)));
+        r->pairCap = grow(r->pairCap, c[1]);
     }
     if (c[2] & lrt::kErrTimeout) r->asyncTimeouts += 1;
     r->debug.visible = c[0];
@@ -1011,12 +1025,11 @@ static int settle_pending_frame(lrt_rast* r) {
     const uint32_t pairs = r->hostCounters[1], status = r->hostCounters[2];
     r->trainPairs = std::min(pairs, r->pairCap);
     r->trainSeenPairs = pairs;
-    r->seenPairs = pairs;
-    r->seenSlots = r->trainParams.count;
+    note_counts(r, r->hostCounters, r->trainParams.count);
     r->debug.pairs_count = std::min(pairs, r->pairCap);
     r->debug.visible = r->hostCounters[0];
-    if (pairs > r->pairCap || (status & lrt::kErrOverflow) != 0) {
-        r->pairCap = grow(r->pairCap, std::max(pairs, r->pairCap + 1));
+    if (pairs > r->pairCap || (status & (lrt::kErrOverflow | lrt::kErrRuns | lrt::kErrTooManyPairs)) != 0) {
+        r->pairCap = grow(r->pairCap, pairs);
         r->trainReady = false;
         return fail(r, LRT_OVERFLOW, "the training forward emitted more pairs than its buffer held; "
                                      "the buffers are grown, run the step again");

@@ -138,6 +138,7 @@ __device__ __forceinline__ float splat_power(float4 conic, float dx, float dy) {
 constexpr uint32_t kErrOverflow = 1u;
 constexpr uint32_t kErrTimeout = 2u;
 constexpr uint32_t kErrTooManyPairs = 4u;
+constexpr uint32_t kErrRuns = 8u;   // more runs of tiles than their buffer holds (rows.cu)
 
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 

@@ -204,13 +204,15 @@ depth_runs_kernel(RowFrame f, RowZeroed z, RowScratch s, uint32_t lastBlock) {
         if (tid == 0) sBase[0] = b;
     } else if (tid < 64) {
         const unsigned long long b = frame_lookback(z.runStatus, part, lastBlock, blockRuns, f.counters + 3,
-                                                    f.counters + 2);
+                                                    f.counters + 2, kErrRuns);
         if (tid == 32) sBase[1] = b;
     }
     __syncthreads();
     const uint32_t base = static_cast<uint32_t>(sBase[1]);
+    if (tid == 0 && f.pairOffsets != nullptr && sBase[0] + blockPairs > f.pairCap)   // a training frame: see runs_whole
+        atomicOr(f.counters + 2, kErrOverflow);
     if (sBase[1] + blockRuns > f.runCap) {   // they would not fit: the frame is drawn again
-        if (tid == 0) atomicOr(f.counters + 2, kErrOverflow);
+        if (tid == 0) atomicOr(f.counters + 2, kErrRuns);
         return;
     }
     at += base;
@@ -280,10 +282,11 @@ __device__ __forceinline__ uint32_t strided_lookback(unsigned long long* word, s
 // tile order, the ones left would hold emit indices up to the frame's total,
 // and the backward, which may be enqueued before the counts are read, writes
 // a pair's partials at its emit index. Such a frame gets no pairs (its ranges
-// stay empty) and is reported as overflowed.
+// stay empty) and is reported as overflowed (kErrOverflow, which only a
+// training frame raises before its pairs are written).
 __device__ __forceinline__ bool runs_whole(const RowFrame& f, uint32_t n) {
-    return n != 0 && n <= f.runCap && (f.counters[2] & (kErrTimeout | kErrTooManyPairs)) == 0 &&
-           (f.pairEmit == nullptr || f.counters[1] <= f.pairCap);
+    return n != 0 && n <= f.runCap &&
+           (f.counters[2] & (kErrTimeout | kErrTooManyPairs | kErrRuns | kErrOverflow)) == 0;
 }
 
 // Bound by latency (each run gathers its splat's mask and rectangle from L2)

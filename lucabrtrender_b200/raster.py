@@ -429,6 +429,7 @@ class TileRasterizer:
             "depth_bits": v.depth_bits,
             "tile_bits": v.tile_bits,
             "visible": v.visible,
+            "from_runs": bool(v.from_runs),
         }
 
     def filter3d(self, cloud: GpuSplats, views: Sequence[tuple], coefficient: float = 0.2,

@@ -137,3 +137,122 @@ def test_an_enqueued_training_step_that_outgrows_its_buffer():
     finally:
         r.close()
         fresh.close()
+
+
+def words_handle(n, pairs, width, height):
+    """A handle whose next frame of n splats is made from sorted words: its
+    buffer holds as many pairs, and the last frame it read was of fewer splats."""
+    tiles = -(-width // 16) * -(-height // 16)
+    k = -(-pairs // tiles) + 1
+    assert k != n
+    r = L.TileRasterizer.create(0)
+    sc = scene(k, width, height, 3.0, 0.1, spread=0.1)   # every splat over every tile
+    assert r.render(sc.camera, sc.gpu_instances(), sc.settings, L.RenderTargets()).pairs >= pairs
+    return r
+
+
+# Faint needles thousands of pixels long. A row of tiles of which such a splat
+# touches some with a gap between them makes it a run for every tile of its
+# rectangle: these have 2.3M pairs or more, and several runs for each.
+NEEDLES, NEEDLE_PAIRS, NEEDLE_SIZE = 100_000, 6_000_000, (3840, 2160)
+
+
+def needle_arrays(n=NEEDLES):
+    rng = np.random.default_rng(1)
+    log_scales = np.full((n, 3), -9.0, np.float32)
+    log_scales[:, 0] = 2.0 + 0.3 * rng.standard_normal(n)
+    return (0.5 * rng.standard_normal((n, 3))).astype(np.float32), log_scales, \
+        rng.standard_normal((n, 4)).astype(np.float32), rng.uniform(-5.5, -5.4, n).astype(np.float32)
+
+
+def needles():
+    means, log_scales, quats, logits = needle_arrays()
+    raw = np.zeros((NEEDLES, 14), np.float32)
+    raw[:, 0:3], raw[:, 3], raw[:, 4:7], raw[:, 7:11], raw[:, 11:14] = means, logits, log_scales, quats, means
+    return H.Scene("needles", [(L.pack_splats(raw, 0, 0), np.eye(4), None)], H.camera((0.2, 0.3, 2.5), focal=24.0),
+                   H.settings(*NEEDLE_SIZE))
+
+
+def blobs():
+    """As many splats, of 2^21 pairs and six a splat too, but fewer runs than pairs."""
+    return scene(NEEDLES, *NEEDLE_SIZE, -4.2, 0.3)
+
+
+def draw(r, sc):
+    t = L.RenderTargets()
+    stats = r.render(sc.camera, sc.gpu_instances(), sc.settings, t)
+    assert stats.pairs >= max(MIN_PAIRS, MIN_PER_SPLAT * NEEDLES) and stats.pairs <= NEEDLE_PAIRS, stats.pairs
+    return t.colour.clone(), t.depth.clone(), bool(r.debug_view().from_runs)
+
+
+def test_frames_of_more_runs_than_pairs():
+    """Drawn from sorted words, whether the runs are met with a wait (they do
+    not fit, on the second attempt) or in an enqueued frame that counts them
+    first; one enqueued after a frame that fitted is reported, and drawn again."""
+    sc, fits = needles(), blobs()
+    r, words = L.TileRasterizer.create(0), words_handle(NEEDLES, NEEDLE_PAIRS, *NEEDLE_SIZE)
+    other = L.TileRasterizer.create(0)
+    try:
+        want_colour, want_depth, from_runs = draw(words, sc)
+        assert not from_runs and float(want_colour.abs().max()) > 0.0
+        for _ in range(2):   # runs unknown, then known
+            colour, depth, from_runs = draw(r, sc)
+            assert not from_runs
+            assert torch.equal(colour, want_colour) and torch.equal(depth, want_depth)
+        assert draw(other, fits)[2]
+        for handle, overflows in ((words, False), (other, True)):   # both forms' counts of the frame before
+            t = L.RenderTargets(*NEEDLE_SIZE)
+            instances = sc.gpu_instances()
+            if overflows:
+                fit_instances = fits.gpu_instances()
+                handle.render_async(fits.camera, fit_instances, fits.settings, t)
+                handle.settle()
+                handle.render_async(sc.camera, instances, sc.settings, t)
+                with pytest.raises(L.LrtError) as info:
+                    handle.settle()
+                assert info.value.code == _abi.OVERFLOW
+            for _ in range(3):
+                handle.render_async(sc.camera, instances, sc.settings, t)
+                handle.settle()
+                assert torch.equal(t.colour, want_colour) and torch.equal(t.depth, want_depth)
+    finally:
+        for handle in (r, words, other):
+            handle.close()
+
+
+def test_training_steps_of_more_runs_than_pairs():
+    """The same in training steps: a waited one, and one enqueued after a step
+    whose runs fitted, which is reported by its backward."""
+    means, log_scales, quats, logits = needle_arrays()
+    sh = np.random.default_rng(2).uniform(-0.5, 0.5, (NEEDLES, 16, 3)).astype(np.float16).astype(np.float32)
+    thin = dict(means=means, log_scales=log_scales, quats=quats, logits=logits, sh=sh)
+    wide = dict(thin, log_scales=np.full_like(log_scales, -4.4), logits=np.full_like(logits, -1.0))
+    cam, settings = TF.frame(*NEEDLE_SIZE, eye=(0.2, 0.3, 1.6))
+    target = torch.rand(NEEDLE_SIZE[1], NEEDLE_SIZE[0], 3, generator=torch.Generator().manual_seed(3)).cuda()
+
+    def step(r, p):
+        t = {k: torch.from_numpy(v).cuda().requires_grad_(True) for k, v in p.items()}
+        colour, _ = L.rasterize(t["means"], t["log_scales"], t["quats"], t["logits"], t["sh"], cam, settings, r)
+        L.l1_loss(colour, target, r).backward()
+        return [colour.detach()] + [v.grad for v in t.values()], bool(r.debug_view().from_runs)
+
+    r, words = L.TileRasterizer.create(0), words_handle(NEEDLES, NEEDLE_PAIRS, *NEEDLE_SIZE)
+    waited = L.TileRasterizer.create(0)
+    try:
+        want, from_runs = step(words, thin)
+        assert not from_runs and float(want[0].abs().max()) > 0.0
+        for _ in range(2):
+            got, from_runs = step(waited, thin)
+            assert not from_runs
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        for _ in range(3):
+            assert step(r, wide)[1]
+        with pytest.raises(L.LrtError) as info:
+            step(r, thin)
+        assert info.value.code == _abi.OVERFLOW
+        got, from_runs = step(r, thin)
+        assert not from_runs
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    finally:
+        for handle in (r, words, waited):
+            handle.close()
