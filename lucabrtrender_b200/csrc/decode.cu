@@ -291,11 +291,14 @@ cudaError_t launch_decode_splats(const float* raw, uint32_t count, const lrt_spl
     uint32_t* tail = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + decode_status_bytes(count) - 16);
     // Stage the records through shared memory when a block's fit (and the
     // records start 16-byte aligned); otherwise read them in place.
+    constexpr size_t kStageMost = 160 * 1024;
     const size_t smem = size_t{kDecodeThreads} * e.floats_per_record * sizeof(float);
-    const bool stage = smem <= 160 * 1024 && (reinterpret_cast<uintptr_t>(raw) & 15u) == 0;
+    const bool stage = smem <= kStageMost && (reinterpret_cast<uintptr_t>(raw) & 15u) == 0;
     if (stage) {
+        // Always the most: the limit belongs to the process, and another
+        // thread may be about to decode longer records.
         const cudaError_t a = cudaFuncSetAttribute(decode_splats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(smem));
+                                                   static_cast<int>(kStageMost));
         if (a != cudaSuccess) return a;
     }
     decode_splats_kernel<<<blocks, kDecodeThreads, stage ? smem : 0, stream>>>(

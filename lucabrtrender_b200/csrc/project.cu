@@ -1221,6 +1221,25 @@ emit_pairs_kernel(uint32_t n, const ProjRecord* __restrict__ proj, const uint4* 
     }
 }
 
+// The staged harmonics' shared memory: up to 24 words a splat (degree 3 and,
+// in training, the base colour) it fits the 48 KB a launch may take beside the
+// kernel's own 19 KB. Longer rows raise the kernel's limit to the most the
+// device gives, never to their own size: the limit belongs to the process,
+// and another thread may be about to launch the same kernel with longer ones.
+template <class Kernel>
+cudaError_t allow_staged(Kernel kernel, size_t smem) {
+    if (smem <= size_t{kProjectThreads} * 24 * 4) return cudaSuccess;
+    cudaFuncAttributes own;
+    cudaError_t e = cudaFuncGetAttributes(&own, kernel);
+    if (e != cudaSuccess) return e;
+    int device = 0, most = 0;
+    if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - static_cast<int>(own.sharedSizeBytes));
+}
+
 template <class Src>
 cudaError_t launch(const FrameParams& f, const FrameParams* fDev, const Src& src, TrainOutputs train, bool stage,
                    ProjRecord* proj, uint4* rects,
@@ -1230,8 +1249,7 @@ cudaError_t launch(const FrameParams& f, const FrameParams* fDev, const Src& src
     const uint32_t stageWords = stage ? f.shWords : 0u;
     const uint32_t shVector = (reinterpret_cast<uintptr_t>(src.sh) & 15u) == 0 ? 1u : 0u;
     const size_t smem = stage ? size_t{kProjectThreads} * f.shWords * 4 : 0;
-    cudaError_t e = cudaFuncSetAttribute(project_emit_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(std::max<size_t>(smem, 1)));
+    const cudaError_t e = allow_staged(project_emit_kernel<Src>, smem);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = project_partitions(f.count);
     project_emit_kernel<Src><<<blocks, kProjectThreads, smem, stream>>>(
@@ -1253,8 +1271,7 @@ cudaError_t launch_only(const FrameParams& f, const Src& src, bool stage, ProjRe
     const auto chained = runs ? project_emit_kernel<Src, false, true, true> : project_emit_kernel<Src, false, true, false>;
     const auto plain = runs ? project_emit_kernel<Src, false, false, true> : project_emit_kernel<Src, false, false, false>;
     for (auto kernel : {chained, plain}) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(std::max<size_t>(smem, 1)));
+        const cudaError_t e = allow_staged(kernel, smem);
         if (e != cudaSuccess) return e;
     }
     const uint32_t blocks = project_partitions(f.count);

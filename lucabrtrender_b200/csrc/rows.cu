@@ -58,6 +58,10 @@ static_assert(kTilesPerSpread * kRunTile == kSpreadRuns, "a spread holds whole t
 // of eight tiles (a lane's two 16-byte accesses), and four more, which puts
 // the 32 rows' words of one tile on eight banks.
 __host__ __device__ constexpr uint32_t spread_stride(uint32_t tilesX) { return ((tilesX + 7u) & ~7u) + 4u; }
+// row_pairs_kernel's dynamic shared memory.
+constexpr size_t spread_bytes(uint32_t tilesX, bool train) {
+    return (kSpreadWords * spread_stride(tilesX) + kSpreadRuns * (train ? 2u : 1u)) * sizeof(uint32_t);
+}
 constexpr uint32_t kOffsetItems = 8;                    // depth positions a thread of depth_runs_kernel takes
 static_assert(kRowThreads == kProjectThreads && kRowThreads == kMaxBands, "a thread a tile row, the scans' block size");
 
@@ -759,17 +763,19 @@ cudaError_t launch_row_pairs(const RowFrame& f, cudaStream_t stream) {
     cudaError_t e = launch_chained(row_counts_kernel<true>, row_counts_kernel<false>, dim3(std::min(most, 148u * 8u)),
                                    dim3(kRowThreads), 0, stream, f, z, s);
     if (e != cudaSuccess) return e;
-    const size_t smem = (kSpreadWords * spread_stride(f.tilesX) + kSpreadRuns * (f.pairEmit != nullptr ? 2u : 1u)) *
-                        sizeof(uint32_t);
+    const size_t smem = spread_bytes(f.tilesX, f.pairEmit != nullptr);
     // As many blocks as the SMs hold at once: the dynamic shared memory, the
     // kernel's own and 1 KB a block, of 228 KB; 2048 threads.
     constexpr size_t kOwn = sizeof(SpreadPlan) + (2 * kMaxBands + 2) * sizeof(uint32_t) + 1024;
     const uint32_t perSm = static_cast<uint32_t>(std::min<size_t>(2048 / kSpreadThreads, (228u << 10) / (smem + kOwn)));
     const dim3 grid(std::min(most, 148u * perSm));
     auto launch = [&](auto chained, auto plain) -> cudaError_t {
+        // The limit belongs to the process, and a thread with another handle
+        // may be between these lines with a frame of another width: always
+        // the widest frame's.
         for (auto kernel : {chained, plain}) {
-            const cudaError_t a =
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            const cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(spread_bytes(kMaxBands, true)));
             if (a != cudaSuccess) return a;
         }
         return launch_chained(chained, plain, grid, dim3(kSpreadThreads), smem, stream, f, z, s);
