@@ -136,6 +136,10 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     }
     const uint32_t launches = static_cast<uint32_t>(clouds.size());
     if (total > 0xFFFFFFFFull) return fail(r, LRT_UNSUPPORTED, "more than 2^32 splats in one frame");
+    // Any frame, enqueued ones included, overwrites what a training forward
+    // left for its backward.
+    r->trainReady = false;
+    r->trainPending = false;
     DeviceScope scope(r->device);
     cudaStream_t stream = static_cast<cudaStream_t>(streamPtr);
     // The handle's buffers serve one frame at a time: a frame on another
@@ -524,8 +528,6 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     r->debug.tile_bits = tileBits;
     r->debug.from_runs = byRows ? 1u : 0u;
     r->debug.visible = visible;
-    r->trainReady = false;
-    r->trainPending = false;
     if (train) {
         r->trainFrame = lastParams;
         r->trainBlend = bp;
@@ -1567,6 +1569,10 @@ extern "C" int lrt_rast_render_batch(lrt_rast* r, const lrt_splat_instance* inst
         return fail(r, LRT_OVERFLOW, "pair capacity exceeded");
     };
 
+    // The batch reuses the pair buffers: a training forward still waiting for
+    // its backward is dropped.
+    r->trainReady = false;
+    r->trainPending = false;
     LRT_CUDA(r, cudaEventRecord(B.in, caller), "event");
     LRT_CUDA(r, cudaStreamWaitEvent(B.stream, B.in, 0), "event");
     if (r->frameDoneSet) LRT_CUDA(r, cudaStreamWaitEvent(B.stream, r->frameDone, 0), "frame order");

@@ -242,3 +242,35 @@ def test_an_fp16_working_copy_of_the_coefficients_gives_the_same_step(rasterizer
     with pytest.raises(ValueError):
         L.rasterize(t["means"], t["log_scales"], t["quats"], t["logits"], t["sh"], cam, settings, rasterizer,
                     sh_storage=t["sh"].detach())
+
+
+@pytest.mark.parametrize("between", ["render", "render_async", "render_batch"])
+def test_a_render_drops_the_forward_that_waits_for_its_backward(between):
+    """The frame's buffers are the ones the backward would read: it is refused
+    after any render in between, enqueued ones and batches included."""
+    from lucabrtrender_b200 import _abi
+    import helpers as H
+    scene = H.synthetic_scene(3000, 96, 96, seed=51)
+    instances, targets = scene.gpu_instances(), L.RenderTargets(96, 96)
+    p = TF.make_params(3000, 52)
+    cam, settings = TF.frame(96, 96)
+    raster = L.TileRasterizer.create(0)
+    try:
+        for _ in range(2):   # sizes the buffers: the frames below are enqueued
+            raster.render(scene.camera, instances, scene.settings, targets)
+            gpu_forward(raster, p, cam, settings)
+            raster.debug_view()
+        _, colour, _ = gpu_forward(raster, p, cam, settings, requires_grad=True)
+        if between == "render_batch":
+            raster.render_batch([(scene.camera, 96, 96)] * 2, instances, scene.settings)
+        else:
+            getattr(raster, between)(scene.camera, instances, scene.settings, targets)
+        with pytest.raises(L.LrtError) as info:
+            colour.sum().backward()
+        assert info.value.code == _abi.INVALID_ARGUMENT
+        raster.settle()
+        t, colour, _ = gpu_forward(raster, p, cam, settings, requires_grad=True)
+        colour.sum().backward()
+        assert all(v.grad is not None for v in t.values())
+    finally:
+        raster.close()
