@@ -99,7 +99,7 @@ struct RowFrame {
     uint32_t* counters;            // [1] pairs, [2] error bits, [4] runs
     uint32_t* pairOffsets;         // out, training frames: each slot's first emit index (else null)
     uint64_t* runs;                // runCap sorted runs
-    uint32_t* runEmit;             // training frames: their first emit index (else null)
+    uint32_t* runEmit;             // training frames: runCap first emit indices (else null)
     uint32_t runCap, pairCap;
     uint32_t* pairSlots;           // out: every tile's slots
     uint32_t* pairEmit;            // out, training frames: the pairs' emit indices (else null)

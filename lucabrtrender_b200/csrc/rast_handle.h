@@ -30,7 +30,10 @@ struct lrt_rast {
     int device = 0;
     std::string error;
     DeviceBuffer proj, rects, touched, keys;            // per slot
-    DeviceBuffer pairs, pairsAlt;                        // per pair
+    // Per pair, 8 bytes each: the pair words and the sort's other buffer; in
+    // frames made from runs (rows.cu) the runs, and every tile's slots followed
+    // by their emit indices.
+    DeviceBuffer pairs, pairsAlt;
     DeviceBuffer ranges;                                 // per tile
     DeviceBuffer tileOrder;                              // per tile: the blend's launch order
     DeviceBuffer scanScratch, sortScratch;               // look-back status words, tickets
@@ -38,9 +41,10 @@ struct lrt_rast {
     DeviceBuffer algoKeysAlt, algoValsAlt;               // lrt_radix_sort's ping-pong buffers
     DeviceBuffer depthWords, depthWordsAlt, splatAux;    // per slot: depth words (two-step frames), aux words
     DeviceBuffer rowTable;                               // large splats' rows (first column, count)
-    DeviceBuffer runCounts, runs, runEmit, rowScratch;   // rows.cu: per slot, per run (and its first emit index), scratch
-    DeviceBuffer pairSlots, pairEmit;                    // rows.cu: every tile's slots (and, training, emit indices)
-    const uint32_t* debugLow = nullptr;                  // what the last frame's pair words hold below the tile (rows.cu)
+    DeviceBuffer runCounts, rowScratch;                  // rows.cu: per slot, scratch
+    // The last frame made from runs: where in pairsAlt, in 32-bit words, its
+    // pairs' low fields begin (the slots, or a training frame's emit indices).
+    size_t debugLow = 0;
     uint32_t rowCap = 0;                                 // its entries
     lrt::SortFault sortFault;                            // lrt_radix_sort's planted fault (tests only)
     DeviceBuffer filterCameras, filterScratch;           // lrt_rast_filter3d's cameras and lowest rate

@@ -66,7 +66,7 @@ void lrt_rast_destroy(lrt_rast* r) {
     for (DeviceBuffer* b : {&r->proj, &r->rects, &r->touched, &r->keys, &r->pairs, &r->pairsAlt,
                             &r->ranges, &r->scanScratch, &r->sortScratch, &r->counters, &r->algoKeysAlt,
                             &r->algoValsAlt, &r->depthWords, &r->depthWordsAlt, &r->splatAux, &r->rowTable,
-                            &r->runCounts, &r->runs, &r->runEmit, &r->rowScratch, &r->pairSlots, &r->pairEmit,
+                            &r->runCounts, &r->rowScratch,
                             &r->pairValues, &r->pairValuesAlt, &r->pairOffsets, &r->pixState, &r->pixLast, &r->partials, &r->metricScratch, &r->lossScratch, &r->trainBatchGrad,
                             &r->trainBatchViews, &r->trainBatchLoss, &r->lodBuild.globals,
                             &r->lodBuild.partial, &r->lodBuild.keys, &r->lodBuild.keysAlt, &r->lodBuild.order,
@@ -267,24 +267,17 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         RowFrame rows{};
         if (countRuns) LRT_CUDA(r, ensure(r->runCounts, size_t{r->splatCap} * sizeof(uint2)), "run counts");
         if (byRows) {
-            // Room for a run a pair, and a quarter more.
-            rows.runCap = static_cast<uint32_t>(
-                std::min<uint64_t>(uint64_t{r->pairCap} + r->pairCap / 4 + 1024, 0xFFFFF000ull));
+            rows.runCap = std::min(r->pairCap, 0xFFFFF000u);   // room for a run a pair
             rows.pairCap = r->pairCap;
-            LRT_CUDA(r, ensure(r->runs, size_t{rows.runCap} * 8), "runs");
-            LRT_CUDA(r, ensure(r->pairSlots, size_t{r->pairCap} * 4), "pairs");
             LRT_CUDA(r, ensure(r->rowScratch, lrt::row_scratch_bytes(slots, rows.runCap, tilesX)), "row scratch");
-            if (train) {
-                LRT_CUDA(r, ensure(r->runEmit, size_t{rows.runCap} * 4), "runs");
-                LRT_CUDA(r, ensure(r->pairEmit, size_t{r->pairCap} * 4), "pairs");
-            }
-        } else {
-            LRT_CUDA(r, ensure(r->pairs, size_t{r->pairCap} * 8), "pairs");
-            LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * 8), "pairs");
-            if (train) {
-                LRT_CUDA(r, ensure(r->pairValues, size_t{r->pairCap} * 4), "pair values");
-                if (!lowIsEmit) LRT_CUDA(r, ensure(r->pairValuesAlt, size_t{r->pairCap} * 4), "pair values");
-            }
+        }
+        // Both forms use the same buffers, so that a handle that draws both
+        // holds them once.
+        LRT_CUDA(r, ensure(r->pairs, size_t{r->pairCap} * 8), "pairs");
+        LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * 8), "pairs");
+        if (train) {
+            LRT_CUDA(r, ensure(r->pairValues, size_t{r->pairCap} * 4), "pair values");
+            if (!lowIsEmit && !byRows) LRT_CUDA(r, ensure(r->pairValuesAlt, size_t{r->pairCap} * 4), "pair values");
         }
         // The two sorts' scratch side by side, so that one launch clears it
         // with the counters, the projection's scratch and the tile ranges.
@@ -376,10 +369,10 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             rows.bands = bands;
             rows.counters = counters;
             rows.pairOffsets = train ? static_cast<uint32_t*>(r->pairOffsets.ptr) : nullptr;
-            rows.runs = static_cast<uint64_t*>(r->runs.ptr);
-            rows.runEmit = train ? static_cast<uint32_t*>(r->runEmit.ptr) : nullptr;
-            rows.pairSlots = static_cast<uint32_t*>(r->pairSlots.ptr);
-            rows.pairEmit = train ? static_cast<uint32_t*>(r->pairEmit.ptr) : nullptr;
+            rows.runs = pairBuf;
+            rows.runEmit = train ? static_cast<uint32_t*>(r->pairValues.ptr) : nullptr;
+            rows.pairSlots = static_cast<uint32_t*>(r->pairsAlt.ptr);
+            rows.pairEmit = train ? rows.pairSlots + r->pairCap : nullptr;
             rows.ranges = static_cast<uint2*>(r->ranges.ptr);
             rows.zeroed = static_cast<char*>(r->scanScratch.ptr) + rowsAt;
             rows.scratch = r->rowScratch.ptr;
@@ -390,7 +383,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
             bp.pairShift = 0;
             sorted = reinterpret_cast<const uint64_t*>(rows.pairSlots);
             sortedValues = rows.pairEmit;
-            r->debugLow = lowIsEmit ? rows.pairEmit : rows.pairSlots;
+            r->debugLow = lowIsEmit ? r->pairCap : 0;
         } else {
             bp.pairShift = 1;
             // --- pairs in depth order ----------------------------------------------------------
@@ -417,7 +410,6 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
                      lrt::launch_ranges(sorted, counters + 1, r->pairCap, 32, static_cast<uint2*>(r->ranges.ptr), tiles,
                                         stream, true),
                      "ranges");
-            r->debugLow = nullptr;
         }
         // The blend takes the tiles busiest first, where they outnumber the
         // blocks that start at once.
@@ -1145,14 +1137,15 @@ int lrt_rast_debug_view(lrt_rast* r, lrt_debug_view* out) {
         if (code != LRT_OK) return code;
     }
     *out = r->debug;
-    if (r->debugLow != nullptr && out->pairs == nullptr && out->tiles != 0) {
+    if (out->from_runs != 0 && out->pairs == nullptr && out->tiles != 0) {
         // Frames made from runs keep every tile's slots, not pair words: they
-        // are put together here, where they are looked at.
+        // are put together here, where they are looked at, in the runs' place.
         DeviceScope scope(r->device);
         LRT_CUDA(r, ensure(r->pairs, std::max<size_t>(size_t{out->pairs_count} * 8, 16)), "pair words");
         LRT_CUDA(r,
-                 lrt::launch_pair_words(static_cast<const uint2*>(out->ranges), r->debugLow, out->tiles, out->pairs_count,
-                                        static_cast<uint64_t*>(r->pairs.ptr), nullptr),
+                 lrt::launch_pair_words(static_cast<const uint2*>(out->ranges),
+                                        static_cast<const uint32_t*>(r->pairsAlt.ptr) + r->debugLow, out->tiles,
+                                        out->pairs_count, static_cast<uint64_t*>(r->pairs.ptr), nullptr),
                  "pair words");
         LRT_CUDA(r, cudaStreamSynchronize(nullptr), "pair words");
         out->pairs = r->pairs.ptr;
