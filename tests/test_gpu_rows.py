@@ -4,7 +4,8 @@ oracle bit for bit: the widest and tallest frames that take this form and the
 first ones past it, splats from a few tiles (tile masks) to the whole frame
 (kept rows, and rows planned again where the first frame's table is too
 small), a tile row's runs around the number one block sorts or spreads
-(2048), training frames, and frames that outgrow their buffers."""
+(2048), training frames, frames that outgrow their buffers or have more runs
+than pairs, and every kind of frame that takes this form."""
 from __future__ import annotations
 
 import numpy as np
@@ -18,10 +19,11 @@ import oracle as ora
 import train_fixtures as TF
 from test_gpu_blend_cells import cloud
 from test_gpu_parity import check_parity
+from test_gpu_points import check_frame
 
 pytestmark = pytest.mark.gpu
 
-MIN_PAIRS, MIN_PER_SPLAT = 1 << 21, 6
+MIN_PAIRS, MIN_PER_SPLAT, MAX_SIDE = 1 << 21, 6, 4096
 
 
 def scene(n, width, height, log_scale, sigma=0.5, spread=1.0, eye=(0.2, 0.3, 4.0), opacity=-1.0, focal=24.0):
@@ -29,17 +31,19 @@ def scene(n, width, height, log_scale, sigma=0.5, spread=1.0, eye=(0.2, 0.3, 4.0
                    H.camera(eye, focal=focal), H.settings(width, height))
 
 
-def check(sc, rasterizer=None):
-    """Twice: the first frame's counts choose the form of the second."""
-    r = rasterizer or L.TileRasterizer.create(0)
+def check(sc):
+    """Twice: the first frame's pairs do not fit the buffer of a fresh handle,
+    and it is drawn again in the form its counts choose; the second's form is
+    known before it starts."""
+    r = L.TileRasterizer.create(0)
     try:
         ref = sc.oracle_render()
         assert ref["pairs"] >= MIN_PAIRS and ref["pairs"] >= MIN_PER_SPLAT * ref["slots"], ref["pairs"]
         for _ in range(2):
-            check_parity(r, sc, ref)
+            dbg = check_parity(r, sc, ref)[2]
+            assert dbg["from_runs"] == (max(sc.settings.width, sc.settings.height) <= MAX_SIDE)
     finally:
-        if rasterizer is None:
-            r.close()
+        r.close()
 
 
 @pytest.mark.parametrize("n,width,height", [(4000, 4096, 48), (4000, 4097, 48), (24000, 48, 4096), (24000, 48, 4097),
@@ -59,29 +63,41 @@ def test_splat_sizes(n, log_scale, sigma):
     check(scene(n, 1500, 1100, log_scale, sigma))
 
 
+def words_handle(n, pairs, width, height):
+    """A handle whose next frame of n splats is made from sorted words: its
+    buffer holds as many pairs, and the last frame it read was of fewer splats."""
+    tiles = -(-width // 16) * -(-height // 16)
+    k = -(-pairs // tiles) + 1
+    assert k != n
+    r = L.TileRasterizer.create(0)
+    sc = scene(k, width, height, 3.0, 0.1, spread=0.1)   # every splat over every tile
+    assert r.render(sc.camera, sc.gpu_instances(), sc.settings, L.RenderTargets()).pairs >= pairs
+    return r
+
+
 def test_training_frames():
-    """The forward bit for bit, and the same gradients as the frame made from sorted words."""
+    """The forward against the oracle from both forms, and the same gradients."""
     n, width, height = 30000, 800, 640
     p = TF.make_params(n, 3, log_scale_mean=-1.7, log_scale_sigma=0.8)
     cam, settings = TF.frame(width, height)
     target = torch.rand(height, width, 3, generator=torch.Generator().manual_seed(1)).cuda()
     ref = ora.train_render(L.projection_for(cam, width, height).struct(), TF.raw_cloud(p), settings.struct())
-    r = L.TileRasterizer.create(0)
+    r = words_handle(n, 8_000_000, width, height)
     try:
         grads = []
-        for _ in range(2):
+        for from_runs in (False, False, True):   # words; words, their runs counted; runs
             t = {k: torch.from_numpy(v).cuda().requires_grad_(True) for k, v in p.items()}
             colour, depth = L.rasterize(t["means"], t["log_scales"], t["quats"], t["logits"], t["sh"], cam, settings, r)
             dbg = r.debug_arrays()
-            assert dbg["pairs"].numel() >= max(MIN_PAIRS, MIN_PER_SPLAT * n)
+            assert dbg["pairs"].numel() >= max(MIN_PAIRS, MIN_PER_SPLAT * n) and dbg["from_runs"] == from_runs
             assert np.array_equal(dbg["ranges"].cpu().numpy().view(np.uint32), ref["ranges"])
             assert np.abs(colour.detach().cpu().numpy() - ref["colour"]).max() <= 1e-5
             assert np.abs(depth.cpu().numpy() - ref["depth"]).max() <= 1e-5
             L.l1_loss(colour, target, r).backward()
             grads.append([v.grad.clone() for v in t.values()])
         # A splat's partials stand in the same order either way, so its sums are the same.
-        for a, b in zip(*grads):
-            assert torch.equal(a, b)
+        for a, *others in zip(*grads):
+            assert all(torch.equal(a, b) for b in others)
     finally:
         r.close()
 
@@ -98,10 +114,12 @@ def test_enqueued_frames_that_outgrow_their_buffers():
         r.settle()
         want = near.oracle_render()
         assert first.pairs >= max(MIN_PAIRS, MIN_PER_SPLAT * first.splats) and want["pairs"] > 2 * first.pairs
+        assert r.debug_view().from_runs
         r.render_async(near.camera, instances, near.settings, targets)
         with pytest.raises(L.LrtError):
             r.settle()
         r.render(near.camera, instances, near.settings, targets)
+        assert r.debug_view().from_runs
         assert np.array_equal(targets.colour.cpu().numpy().view(np.uint32), want["colour"].view(np.uint32))
     finally:
         r.close()
@@ -128,7 +146,8 @@ def test_an_enqueued_training_step_that_outgrows_its_buffer():
     try:
         for _ in range(3):   # the first sizes the buffers, the second leaves a quarter free, the third is enqueued
             step(r, far)
-        assert r.debug_arrays()["pairs"].numel() >= max(MIN_PAIRS, MIN_PER_SPLAT * n)
+        dbg = r.debug_arrays()
+        assert dbg["pairs"].numel() >= max(MIN_PAIRS, MIN_PER_SPLAT * n) and dbg["from_runs"]
         with pytest.raises(L.LrtError) as info:
             step(r, near)
         assert info.value.code == _abi.OVERFLOW
@@ -137,18 +156,6 @@ def test_an_enqueued_training_step_that_outgrows_its_buffer():
     finally:
         r.close()
         fresh.close()
-
-
-def words_handle(n, pairs, width, height):
-    """A handle whose next frame of n splats is made from sorted words: its
-    buffer holds as many pairs, and the last frame it read was of fewer splats."""
-    tiles = -(-width // 16) * -(-height // 16)
-    k = -(-pairs // tiles) + 1
-    assert k != n
-    r = L.TileRasterizer.create(0)
-    sc = scene(k, width, height, 3.0, 0.1, spread=0.1)   # every splat over every tile
-    assert r.render(sc.camera, sc.gpu_instances(), sc.settings, L.RenderTargets()).pairs >= pairs
-    return r
 
 
 # Faint needles thousands of pixels long. A row of tiles of which such a splat
@@ -256,3 +263,46 @@ def test_training_steps_of_more_runs_than_pairs():
     finally:
         for handle in (r, words, waited):
             handle.close()
+
+
+@pytest.mark.parametrize("kind", ["instances", "edit", "threshold", "orthographic", "discs", "discs-under"])
+def test_other_frames(kind):
+    """What a frame may hold besides one cloud seen in perspective, against the
+    oracle, bit for bit: instances, an edit, the threshold depth, a parallel
+    projection, discs, and a layer under the splats."""
+    sc = scene(20000, 1200, 900, -2.5, 0.8)
+    packed = sc.clouds[0][0]
+    if kind == "instances":
+        sc.clouds.append((cloud(7000, 3, 0.7, -2.0, 0.5), H.translation((0.4, -0.2, 0.5)) @ H.rotation_y(35.0), None))
+    elif kind == "edit":
+        edit = L.SplatEdit(active=True, centre=(0.1, 0.0, 0.2), size=(1.5, 1.2, 1.4), tint=(1.0, 0.6, 0.3),
+                           opacity=0.7, brightness=1.2)
+        sc.clouds[0] = (packed, np.eye(4), edit)
+    elif kind == "threshold":
+        sc.settings.depth = L.Depth(1)
+    elif kind == "orthographic":
+        sc.camera = H.camera((0.2, 0.3, 4.0), focal=7.0, orthographic=True)
+    pr, style = sc.projection(), L.PointStyle(size_mode=1, size=40.0)
+    packed_points = L.pack_points(ora.random_points(2000, 6), 2)
+    points = [L.PointInstance(L.points_to_device(packed_points), np.eye(4), style)] if "discs" in kind else []
+    host_points = [(ora.HostPoints(packed_points.positions, packed_points.colours), np.eye(4),
+                    H.point_style(1, 40.0))] if points else []
+    under = under_host = None
+    if "under" in kind:
+        under = L.RenderTargets(sc.settings.width, sc.settings.height)
+        gen = torch.Generator().manual_seed(4)
+        shape = (sc.settings.height, sc.settings.width)
+        under.colour.copy_(torch.rand((*shape, 4), generator=gen))
+        depth = 2.0 + 4.0 * torch.rand(shape, generator=gen)
+        under.depth.copy_(torch.where(torch.rand(shape, generator=gen) < 0.3, torch.zeros(shape), depth))
+        under_host = (under.colour.cpu().numpy(), under.depth.cpu().numpy())
+    ref = ora.render(pr.struct(), sc.oracle_instances(), sc.settings.struct(), points=host_points, under=under_host)
+    assert ref["pairs"] >= MIN_PAIRS and ref["pairs"] >= MIN_PER_SPLAT * ref["slots"], (ref["pairs"], ref["slots"])
+    r, targets, instances = L.TileRasterizer.create(0), L.RenderTargets(), sc.gpu_instances()
+    try:
+        for _ in range(2):
+            out = r.render(pr, instances, sc.settings, targets, points=points, under=under)
+            check_frame(r, out, ref, targets)
+            assert r.debug_view().from_runs
+    finally:
+        r.close()
