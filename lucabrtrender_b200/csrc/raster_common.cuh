@@ -140,7 +140,7 @@ constexpr uint32_t kErrTimeout = 2u;
 constexpr uint32_t kErrTooManyPairs = 4u;
 constexpr uint32_t kErrRuns = 8u;   // more runs of tiles than their buffer holds (rows.cu)
 
-__device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
+LRT_HD float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 
 __device__ __forceinline__ float3 to_view(const FrameParams& f, float3 p) {   // frame.slang:91-95
     return make_float3(f.m[0] * p.x + f.m[1] * p.y + f.m[2] * p.z + f.m[3],
@@ -173,8 +173,8 @@ __device__ __forceinline__ float cutoff_power(float alpha) {   // frame.slang:10
 // below its exact one by no more. So when both nearer values are above the
 // gate, cutoff (1 + 64u kappa), every far candidate is above the cutoff too
 // and the answer (false) is the one the four candidates give.
-__device__ __forceinline__ bool power_within_over_box(float a, float b, float c, float lox, float loy, float hix,
-                                                      float hiy, float cutoff, float farGate = INFINITY) {
+LRT_HD bool power_within_over_box(float a, float b, float c, float lox, float loy, float hix, float hiy, float cutoff,
+                                  float farGate = INFINITY) {
     if (lox <= 0.0f && hix >= 0.0f && loy <= 0.0f && hiy >= 0.0f) return 0.0f <= cutoff;
     const bool xNearHi = fabsf(hix) < fabsf(lox), yNearHi = fabsf(hiy) < fabsf(loy);
     bool nearAbove = true;
@@ -202,7 +202,7 @@ __device__ __forceinline__ bool power_within_over_box(float a, float b, float c,
 // The gate for power_within_over_box: infinite (never used) unless the conic
 // is positive definite with kappa <= 1e4 and both stationary points are
 // computed (a, c > 1e-12).
-__device__ __forceinline__ float far_edge_gate(float a, float b, float c, float cutoff) {
+LRT_HD float far_edge_gate(float a, float b, float c, float cutoff) {
     if (!(a > 1e-12f) || !(c > 1e-12f) || !(cutoff >= 0.0f)) return INFINITY;
     const float lmin = 0.5f * (a + c) - sqrtf(0.25f * (a - c) * (a - c) + b * b);
     if (!(lmin > 0.0f)) return INFINITY;
@@ -212,9 +212,8 @@ __device__ __forceinline__ float far_edge_gate(float a, float b, float c, float 
 }
 
 // frame.slang:133-138: does tile (tx, ty) hold a pixel centre inside the footprint?
-__device__ __forceinline__ bool tile_touched(uint32_t width, uint32_t height, float cx, float cy,
-                                             float ca, float cb, float cc, float cutoff, uint32_t tx,
-                                             uint32_t ty, float farGate = INFINITY) {
+LRT_HD bool tile_touched(uint32_t width, uint32_t height, float cx, float cy, float ca, float cb, float cc,
+                         float cutoff, uint32_t tx, uint32_t ty, float farGate = INFINITY) {
     const float firstX = static_cast<float>(tx * kTile) + 0.5f;
     const float firstY = static_cast<float>(ty * kTile) + 0.5f;
     const float lastX = static_cast<float>(min((tx + 1) * kTile, width) - 1) + 0.5f;
@@ -237,14 +236,14 @@ struct TileTest {
     float slopeX, slopeY;   // -b / a and -b / c
     float sure, gate;
 };
-__device__ __forceinline__ TileTest tile_test(float a, float b, float c, float cutoff) {
+LRT_HD TileTest tile_test(float a, float b, float c, float cutoff) {
     const float gate = far_edge_gate(a, b, c, cutoff);
     const bool usual = gate < INFINITY;
     return {usual ? -b / a : 0.0f, usual ? -b / c : 0.0f, usual ? cutoff - (gate - cutoff) : -INFINITY, gate};
 }
 enum class Touch { kNo, kYes, kUnsure };
-__device__ __forceinline__ Touch tile_touch(uint32_t width, uint32_t height, float cx, float cy, float a, float b,
-                                            float c, const TileTest& t, uint32_t tx, uint32_t ty) {
+LRT_HD Touch tile_touch(uint32_t width, uint32_t height, float cx, float cy, float a, float b, float c,
+                        const TileTest& t, uint32_t tx, uint32_t ty) {
     const float lox = static_cast<float>(tx * kTile) + 0.5f - cx, loy = static_cast<float>(ty * kTile) + 0.5f - cy;
     const float hix = static_cast<float>(min((tx + 1) * kTile, width) - 1) + 0.5f - cx;
     const float hiy = static_cast<float>(min((ty + 1) * kTile, height) - 1) + 0.5f - cy;
@@ -252,8 +251,8 @@ __device__ __forceinline__ Touch tile_touch(uint32_t width, uint32_t height, flo
         return t.gate < INFINITY ? Touch::kYes : Touch::kUnsure;
     const float x = fabsf(hix) < fabsf(lox) ? hix : lox, y = fabsf(hiy) < fabsf(loy) ? hiy : loy;
     const float yx = clampf(x * t.slopeY, loy, hiy), xy = clampf(y * t.slopeX, lox, hix);
-    const float q0 = __fmaf_rn(__fmaf_rn(2.0f * b, yx, a * x), x, c * yx * yx);
-    const float q1 = __fmaf_rn(__fmaf_rn(2.0f * b, xy, c * y), y, a * xy * xy);
+    const float q0 = lrt_fma(lrt_fma(2.0f * b, yx, a * x), x, c * yx * yx);
+    const float q1 = lrt_fma(lrt_fma(2.0f * b, xy, c * y), y, a * xy * xy);
     if (q0 <= t.sure || q1 <= t.sure) return Touch::kYes;
     return q0 > t.gate && q1 > t.gate ? Touch::kNo : Touch::kUnsure;
 }
