@@ -1,5 +1,7 @@
-// What the forward and backward blends share: the block size and the
-// conservative per-record box a warp tests before walking a record.
+// What the forward and backward blends share: the block size, the margin that
+// covers the per-pixel test's rounding, and the conservative shapes made with
+// it: a record's box (the backward's warps test it before they walk a record)
+// and its cells of a tile (the forward's lists).
 #pragma once
 
 #include "raster_common.cuh"
@@ -9,17 +11,12 @@ namespace {
 
 constexpr uint32_t kBlendThreads = 256;
 
-// A box outside which no pixel centre can pass the record's cut, with every
-// rounding of the per-pixel test accounted for, so that skipping a record
-// for a whole warp never changes a pixel. {power <= k} is an ellipse whose
-// bounding half-widths are sqrt(k c / det) and sqrt(k a / det) for the conic
-// (a, b, c). The float power of a pixel can fall below the exact one by at
+// The float power of a pixel can fall below the exact one by at
 // most ~4u (|a| dx^2 + 2|b| |dx dy| + |c| dy^2) <= 4u kappa power with
-// kappa = (|a| + 2|b| + |c|) / lambda_min; det itself carries a relative
-// error up to ~4u (|ac| + b^2) / det. delta bounds both with a factor of 8
-// to spare; the cut is widened to cutoff / (1 - delta) and the half-widths by
-// (1 + delta) plus 1e-3 px. Records where delta is not small are never skipped.
-// The divisions and roots are the hardware's approximate ones (a few 2^-22 of
+// kappa = (|a| + 2|b| + |c|) / lambda_min; det = a c - b^2 itself carries a
+// relative error up to ~4u (|ac| + b^2) / det. delta bounds both with a factor
+// of 8 to spare. False where it is not small (or the conic not one of an
+// ellipse): such a record is never skipped. The divisions and roots are the hardware's approximate ones (a few 2^-22 of
 // relative error; a quotient by more than 2^126 is excluded by the bound on
 // the conic's trace): delta is at least 1.3e-5 and holds a factor of 8, so
 // both bounds still hold.
@@ -28,21 +25,31 @@ __device__ __forceinline__ float approx_sqrt(float v) {
     asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
-__device__ __forceinline__ float4 cull_box(const ProjRecord& rec) {
-    const float a = rec.conic.x, b = rec.conic.y, c = rec.conic.z, cutoff = rec.screen.w;
-    const float det = a * c - b * b;
+__device__ __forceinline__ bool cut_margin(float a, float b, float c, float cutoff, float& det, float& invDet,
+                                           float& delta) {
+    det = a * c - b * b;
     const float half = 0.5f * (a + c);
     const float root = approx_sqrt(0.25f * (a - c) * (a - c) + b * b);
     // root's own error (a few 2^-22 of at most half) taken off lmin.
     const float lmin = half - root - 2.0e-6f * half;
-    const float kInf = 3.0e38f;
-    if (!(det > 0.0f) || !(lmin > 0.0f) || !(cutoff >= 0.0f) || !(half < 1.0e30f))
-        return make_float4(-kInf, kInf, -kInf, kInf);
-    const float invDet = __fdividef(1.0f, det);
+    if (!(det > 0.0f) || !(lmin > 0.0f) || !(cutoff >= 0.0f) || !(half < 1.0e30f)) return false;
+    invDet = __fdividef(1.0f, det);
     const float kappa = __fdividef(fabsf(a) + 2.0f * fabsf(b) + fabsf(c), lmin);
     const float cond = (fabsf(a * c) + b * b) * invDet;
-    const float delta = 32.0f * 5.9604645e-08f * (kappa + cond + 4.0f);
-    if (!(delta < 0.25f)) return make_float4(-kInf, kInf, -kInf, kInf);
+    delta = 32.0f * 5.9604645e-08f * (kappa + cond + 4.0f);
+    return delta < 0.25f;
+}
+
+// A box outside which no pixel centre can pass the record's cut, so that
+// skipping a record for a whole warp never changes a pixel. {power <= k} is an
+// ellipse whose bounding half-widths are sqrt(k c / det) and sqrt(k a / det)
+// for the conic (a, b, c); the cut is widened to cutoff / (1 - delta) and the
+// half-widths by (1 + delta) plus 1e-3 px.
+__device__ __forceinline__ float4 cull_box(const ProjRecord& rec) {
+    const float a = rec.conic.x, b = rec.conic.y, c = rec.conic.z, cutoff = rec.screen.w;
+    const float kInf = 3.0e38f;
+    float det, invDet, delta;
+    if (!cut_margin(a, b, c, cutoff, det, invDet, delta)) return make_float4(-kInf, kInf, -kInf, kInf);
     const float k = __fdividef(cutoff, 1.0f - delta) * invDet;
     const float ex = approx_sqrt(k * c) * (1.0f + delta) + 1e-3f;
     const float ey = approx_sqrt(k * a) * (1.0f + delta) + 1e-3f;
@@ -67,16 +74,8 @@ constexpr uint32_t kCells = 16;
 // bounding box.
 __device__ __forceinline__ uint32_t cells_touched(const ProjRecord& rec, float x0, float y0) {
     const float a = rec.conic.x, b = rec.conic.y, c = rec.conic.z, cutoff = rec.screen.w;
-    const float det = a * c - b * b;
-    const float half = 0.5f * (a + c);
-    const float root = approx_sqrt(0.25f * (a - c) * (a - c) + b * b);
-    const float lmin = half - root - 2.0e-6f * half;   // root's own error taken off
-    if (!(det > 0.0f) || !(lmin > 0.0f) || !(cutoff >= 0.0f) || !(half < 1.0e30f)) return 0xFFFFu;
-    const float invDet = __fdividef(1.0f, det);
-    const float kappa = __fdividef(fabsf(a) + 2.0f * fabsf(b) + fabsf(c), lmin);
-    const float cond = (fabsf(a * c) + b * b) * invDet;
-    const float delta = 32.0f * 5.9604645e-08f * (kappa + cond + 4.0f);
-    if (!(delta < 0.25f)) return 0xFFFFu;
+    float det, invDet, delta;
+    if (!cut_margin(a, b, c, cutoff, det, invDet, delta)) return 0xFFFFu;
     const float k = __fdividef(cutoff, 1.0f - delta) * (1.0f + 4.0f * delta);
     const float ex = approx_sqrt(k * invDet * c) * (1.0f + delta) + 1e-3f;
     const float ey = approx_sqrt(k * invDet * a) * (1.0f + delta) + 1e-3f;

@@ -108,6 +108,7 @@ struct RowFrame {
     void* scratch;                 // row_scratch_bytes(slots, runCap, tilesX)
 };
 constexpr uint32_t kMaxBands = 256;
+constexpr uint32_t kSms = 148;   // a B200's multiprocessors: the persistent grids' unit
 size_t row_zeroed_bytes(uint32_t slots);
 size_t row_scratch_bytes(uint32_t slots, uint32_t runCap, uint32_t tilesX);
 cudaError_t launch_row_runs(const RowFrame& f, cudaStream_t stream);    // the runs, sorted by tile row

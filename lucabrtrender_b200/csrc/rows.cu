@@ -47,6 +47,7 @@ constexpr uint32_t kRowThreads = 256;
 constexpr uint32_t kRowWarps = kRowThreads / 32;
 constexpr uint32_t kRunItems = 8;
 constexpr uint32_t kRunTile = kRowThreads * kRunItems;   // runs a block of row_runs_kernel takes at a time
+constexpr uint32_t kRunBlocks = 4;                       // its blocks an SM (64 registers a thread)
 constexpr uint32_t kSpreadRuns = 2048;                   // runs of a tile row a block spreads at a time
 constexpr uint32_t kSpreadWords = kSpreadRuns / 32;
 constexpr uint32_t kSpreadThreads = 512;
@@ -299,7 +300,7 @@ __device__ __forceinline__ bool runs_whole(const RowFrame& f, uint32_t n) {
 // first run lies in it; each marks its first run's place, and a running
 // maximum over the places gives every run its splat.
 template <bool kTrain, bool kChained>
-__global__ void __launch_bounds__(kRowThreads, 4)
+__global__ void __launch_bounds__(kRowThreads, kRunBlocks)
 row_runs_kernel(RowFrame f, RowZeroed z, RowScratch s) {
     chained_entry<kChained>();
     __shared__ unsigned long long sRun[kRunTile];
@@ -308,7 +309,7 @@ row_runs_kernel(RowFrame f, RowZeroed z, RowScratch s) {
     __shared__ uint32_t sBlockStart[kMaxBands];
     __shared__ uint32_t sGlobal[kMaxBands];
     __shared__ uint32_t sScan[kRowWarps];
-    __shared__ uint32_t sPart, sBefore;
+    __shared__ uint32_t sPart;
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u, warp = tid >> 5;
     const uint32_t n = f.counters[4];
@@ -365,7 +366,7 @@ row_runs_kernel(RowFrame f, RowZeroed z, RowScratch s) {
             for (uint32_t k = 0; k < kRunItems; ++k) sOwner[tid * kRunItems + k] = max(v[k], prior);
             __syncthreads();
         }
-        // The runs, four a thread at a time so that their loads overlap.
+        // The runs, two a thread at a time so that their loads overlap.
         constexpr uint32_t kAtOnce = 2;
 #pragma unroll 1
         for (uint32_t p0 = tid; p0 < here; p0 += kAtOnce * kRowThreads) {
@@ -746,8 +747,7 @@ cudaError_t launch_row_runs(const RowFrame& f, cudaStream_t stream) {
     cudaError_t e = launch_chained(depth_runs_kernel<true>, depth_runs_kernel<false>, dim3(blocks), dim3(kRowThreads),
                                    0, stream, f, z, s, blocks - 1);
     if (e != cudaSuccess) return e;
-    // Six blocks an SM by shared memory (37 KB each).
-    const dim3 grid(std::min(run_tiles(f.runCap), 148u * 6u));
+    const dim3 grid(std::min(run_tiles(f.runCap), kSms * kRunBlocks));
     return f.runEmit != nullptr
                ? launch_chained(row_runs_kernel<true, true>, row_runs_kernel<true, false>, grid, dim3(kRowThreads), 0,
                                 stream, f, z, s)
@@ -760,7 +760,7 @@ cudaError_t launch_row_pairs(const RowFrame& f, cudaStream_t stream) {
     const RowZeroed z = row_zeroed(f);
     const RowScratch s = row_scratch(f);
     const uint32_t most = f.runCap / kSpreadRuns + 1 + f.tilesY;
-    cudaError_t e = launch_chained(row_counts_kernel<true>, row_counts_kernel<false>, dim3(std::min(most, 148u * 8u)),
+    cudaError_t e = launch_chained(row_counts_kernel<true>, row_counts_kernel<false>, dim3(std::min(most, kSms * 8u)),
                                    dim3(kRowThreads), 0, stream, f, z, s);
     if (e != cudaSuccess) return e;
     const size_t smem = spread_bytes(f.tilesX, f.pairEmit != nullptr);
@@ -768,7 +768,7 @@ cudaError_t launch_row_pairs(const RowFrame& f, cudaStream_t stream) {
     // kernel's own and 1 KB a block, of 228 KB; 2048 threads.
     constexpr size_t kOwn = sizeof(SpreadPlan) + (2 * kMaxBands + 2) * sizeof(uint32_t) + 1024;
     const uint32_t perSm = static_cast<uint32_t>(std::min<size_t>(2048 / kSpreadThreads, (228u << 10) / (smem + kOwn)));
-    const dim3 grid(std::min(most, 148u * perSm));
+    const dim3 grid(std::min(most, kSms * perSm));
     auto launch = [&](auto chained, auto plain) -> cudaError_t {
         // The limit belongs to the process, and a thread with another handle
         // may be between these lines with a frame of another width: always
