@@ -148,26 +148,25 @@ __device__ __forceinline__ bool finite(float v) { return fabsf(v) < INFINITY; }
 // place while batch k is walked, and the pair words of batch k+2 are on their
 // way in a register.
 //
-// The walk is bound by instruction issue (90% of the issue slots; its records
-// come from L2 and shared memory), and a splat of the usual size covers a
-// third of the pixels of the 8x8 blocks it touches. So each 4x4 cell walks
-// its own list: a thread marks the cells its record may touch (cells_touched),
-// and each cell's eight threads read 16 records' marks each and write the
-// indices of those that may touch it, in order. A warp walks the lists
-// of its four cells side by side and takes as many steps as its longest list
-// has records (at 1M splats, 1080p: 0.56 steps a pair, against 0.82 visits of
-// 8x8 blocks to records whose bounding box meets them). A lane's two pixels
-// go through a step together in packed single precision, each operation one
-// instruction for both and rounded as the scalar one is, and two records'
-// powers and alphas are formed side by side, since one chain of dependent
-// operations a warp leaves issue slots empty. A pixel that a record does not
-// touch takes part with alpha zero, which leaves its sums and T as they are
-// as long as the record's colour and depth are finite; a batch with one that
-// is not updates pixel by pixel. Against whole 8x8 blocks visiting records
+// The walk is bound by instruction issue and by the FMA pipe, which a packed
+// operation holds for two cycles (1M splats at 1080p: 78% of the issue slots,
+// 55% of the pipe; its records come from L2 and shared memory), and a splat of
+// the usual size covers a third of the pixels of the 8x8 blocks it touches.
+// So each 4x4 cell walks its own list: a thread marks the cells its record may
+// touch (cells_touched), and each cell's eight threads read 16 records' marks
+// each and write the indices of those that may touch it, in order. A warp
+// walks the lists of its four cells side by side and takes as many steps as
+// its longest list has records. A lane's two pixels go through a step together
+// in packed single precision, each operation one instruction for both and
+// rounded as the scalar one is, and two records' powers and alphas are formed
+// side by side, since one chain of dependent operations a warp leaves issue
+// slots empty. A pixel that a record does not touch takes part with alpha
+// zero, which leaves its sums and T as they are as long as the record's colour
+// and depth are finite; a batch with one that is not updates pixel by pixel. Against whole 8x8 blocks visiting records
 // pixel by pixel: 1M splats at 1080p 0.386 -> 0.274 ms, 6M at 4K 1.34 ->
-// 1.00 ms, 100k at 512x512 0.115 -> 0.059 ms; 79 issue slots a pair instead of
-// 98 (a packed operation takes two). Bounds of 7 or 8 blocks an SM, without
-// the few spilled bytes the compiler chooses here, are slower (0.285, 0.283).
+// 1.00 ms, 100k at 512x512 0.115 -> 0.059 ms; 57 warp instructions a pair
+// instead of 94. Bounds of 7 or 8 blocks an SM, without the few spilled bytes
+// the compiler chooses here, are slower (0.285, 0.283).
 // Each pixel runs the reference's loop unchanged over the records it is
 // given, so it stops at T < 1e-4 exactly as the reference does; a warp leaves
 // a batch when no cell of it has records left for pixels still blending, and

@@ -181,7 +181,8 @@ cudaError_t launch_publish_counters(const uint32_t* counters, const uint32_t* ba
 // gain nothing from an order: 192 tiles (3k splats, 250x190) blend 17.0 us in
 // index order and 17.3 busiest first, 294 tiles (a 20k-splat training frame)
 // 57.4 and 56.9, for 3.6 us of ordering (9.8 with the backward's). At 1024
-// tiles (100k, 512x512) an SM's share still matters: 63.6 and 55.8.
+// tiles (100k, 512x512) an SM's share still matters: 63.6 and 55.8. Between
+// 294 and 1024 tiles nothing was measured.
 constexpr uint32_t kOrderMinTiles = 512;
 size_t tile_order_scratch_bytes(uint32_t tiles);
 cudaError_t launch_tile_order(const uint2* ranges, uint32_t tiles, uint32_t* order, uint32_t* scratch,

@@ -22,10 +22,15 @@ namespace lrt {
 // once all of this grid's blocks are running.
 //
 // Chaining is on only inside a ChainScope that asks for it: the frame entry
-// points open one for frames of at least kChainMinPixels, where the overlap
-// was measured to pay (1080p: end to end 1.026 -> 0.957 ms a frame). Smaller
-// frames are bound by the host's launch work, so they (and the batched
-// paths, sorts and everything else) use the ordinary launch.
+// points open one for frames of at least kChainMinPixels; smaller frames, the
+// batched paths, sorts and everything else use the ordinary launch. The line
+// was drawn while six event records stood between a frame's kernels and a
+// chained launch cost a smaller frame more than it gave. Without them, us a
+// call, ordinary / chained: above the line 1M splats at 1080p 632 / 620, a
+// training step of those 1584 / 1559, 6M at 4K 5012 / 5038; below it four
+// frames of 500k at 1279x719 1298 / 1229, 100k at 512x512 185 / 167, 3k at
+// 250x190 110 / 93, a training step of 20k at 333x217 350 / 323, a cut of 1M
+// and its frame (1080p) the same either way. So the line could lie lower now.
 constexpr uint64_t kChainMinPixels = 1920ull * 1080ull;
 inline thread_local bool tChainLaunches = false;
 struct ChainScope {
