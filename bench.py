@@ -43,11 +43,12 @@ L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (read + written) of one launch, from ncu (`dram__bytes_read.sum +
 # dram__bytes_write.sum`) on one frame of this orbit; the capture and its command
 # are summarised under profiles/ (blend_1M_1080p.md).
-PROFILED_DRAM_BYTES = {"blend": 53.549312e6 + 7.519232e6}
-# The blend is bound by instruction issue, not by HBM: its issue-active
+PROFILED_DRAM_BYTES = {"blend": 56.926976e6 + 8.576e6}
+# The blend is bound by instruction issue and the FMA pipe (its packed
+# operations hold it two cycles), not by HBM: its issue-active
 # fraction (`smsp__issue_active.avg.pct_of_peak_sustained_active`) from the
 # same capture, the secondary roofline its HBM fraction is read beside.
-PROFILED_ISSUE_ACTIVE = {"blend": 0.9007}
+PROFILED_ISSUE_ACTIVE = {"blend": 0.7752}
 
 
 def orbit_camera(L, k: int):
@@ -401,13 +402,17 @@ def run_lod(L, torch, stream, raster, cloud, settings, peak) -> dict:
                             "select_ms includes its one count read back"}
 
 
-def sort_bytes(slots: float, pairs: float, tiles: int) -> dict:
+def sort_bytes(slots: float, pairs: float, tiles: int, from_runs: bool = False) -> dict:
     """Algorithmic bytes of a frame's two sorts: the depth sort of one 8-byte
     word per slot on 24 key bits, and the stable sort of one 8-byte word per
     pair on the tile bits; per 8-bit pass 8 B read + 8 B written per word (the
-    digit counts come from the kernels that write the keys)."""
+    digit counts come from the kernels that write the keys). A frame made
+    from the splats' runs of tiles sorts no pairs: of its ordering only the 4
+    bytes written per pair are counted, not the runs."""
     tile_bits = max(1, math.ceil(math.log2(tiles)))
     depth_passes, tile_passes = 3, math.ceil(tile_bits / 8)
+    if from_runs:
+        return {"depth": 16 * depth_passes * slots, "tile": 4 * pairs, "depth_passes": depth_passes, "tile_passes": 0}
     return {"depth": 16 * depth_passes * slots, "tile": 16 * tile_passes * pairs,
             "depth_passes": depth_passes, "tile_passes": tile_passes}
 
@@ -459,10 +464,10 @@ HEAVY_SEED = 7
 def run_sort_heavy(L, torch, dev, raster, peak, clocks, steps: int, splats: int = HEAVY_SPLATS) -> dict:
     """The sort-heavy frame: 6M splats with means N(0,2) and log-scales
     N(-3.5,0.7), 3840x2160, 16x16 tiles, camera 4 units out. Per-stage ms
-    from the frame's own events, pairs, and the pair sort's algorithmic bytes
-    per second against the HBM peak. The cloud is decoded on the device from
+    from the frame's own events, pairs, and the algorithmic bytes per second of
+    what orders them (sort_bytes) against the HBM peak. The cloud is decoded on the device from
     its raw records (the same bytes as the host packing). The working set
-    (about 4 GB of pair words) is far larger than L2, so no flush is needed."""
+    (1 GB of slots by tile, and their runs) is far larger than L2, so no flush is needed."""
     raw = L.synthetic_records(splats, HEAVY_SEED, mean_sigma=2.0, log_scale_mean=-3.5, log_scale_sigma=0.7)
     raw_dev = torch.from_numpy(raw).to(dev)
     del raw
@@ -490,8 +495,10 @@ def run_sort_heavy(L, torch, dev, raster, peak, clocks, steps: int, splats: int 
     clocks.window(w0, time.time())
     pairs = float(np.mean([x.pairs for x in st]))
     tiles = ((HEAVY_WIDTH + 15) // 16) * ((HEAVY_HEIGHT + 15) // 16)
-    sb = sort_bytes(splats, pairs, tiles)
-    sort_ms = float(np.mean([x.depth_sort_ms + x.tile_sort_ms for x in st]))
+    from_runs = bool(raster.debug_view().from_runs)
+    sb = sort_bytes(splats, pairs, tiles, from_runs)
+    # In a frame made from runs the emission stage holds their sort by tile row.
+    sort_ms = float(np.mean([x.depth_sort_ms + x.tile_sort_ms + (x.emit_ms if from_runs else 0.0) for x in st]))
     gbs = (sb["depth"] + sb["tile"]) / (sort_ms * 1e-3) / 1e9
     out = {"workload": f"{splats / 1e6:g}M splats, means N(0,2), log-scales N(-3.5,0.7), 3840x2160, 16x16 tiles, "
                        "eye (0, 0, 4)",
@@ -499,11 +506,16 @@ def run_sort_heavy(L, torch, dev, raster, peak, clocks, steps: int, splats: int 
            "stages_ms": {k: round(float(np.mean([getattr(x, k) for x in st])), 4)
                          for k in ("project_ms", "depth_sort_ms", "emit_ms", "tile_sort_ms", "blend_ms")},
            "pairs": int(pairs), "visible": int(np.mean([x.visible for x in st])),
+           "pair_order": "runs of tiles" if from_runs else "pair words",
            "sort_passes": {"depth": sb["depth_passes"], "tile": sb["tile_passes"]},
-           "sort_bytes": "depth sort: 8 B words per slot, tile sort: 8 B words per pair; per 8-bit pass 8 B read "
-                         "+ 8 B written per word (the digit counts come from the kernels that write the keys); "
-                         "tile_sort_ms also holds the ranges pass",
-           "sort_gbs": round(gbs, 1), "sort_frac_of_hbm": round(gbs / peak, 4)}
+           "sort_bytes": ("depth sort: 8 B words per slot, per 8-bit pass 8 B read + 8 B written per word; the pairs, "
+                          "made from the splats' runs of tiles: 4 B written per pair (the runs not counted); "
+                          "over depth_sort_ms + emit_ms (the runs) + tile_sort_ms (the pairs and ranges)") if from_runs
+                         else ("depth sort: 8 B words per slot, tile sort: 8 B words per pair; per 8-bit pass 8 B read "
+                               "+ 8 B written per word (the digit counts come from the kernels that write the keys); "
+                               "tile_sort_ms also holds the ranges pass"),
+           "sort_gbs": round(gbs, 1), "sort_frac_of_hbm": round(gbs / peak, 4),
+           "gpairs_per_s": round(pairs / sort_ms / 1e6, 1)}
     del cloud, inst, targets
     torch.cuda.empty_cache()
     return out
