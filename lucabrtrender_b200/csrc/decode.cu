@@ -294,7 +294,7 @@ cudaError_t launch_decode_splats(const float* raw, uint32_t count, const lrt_spl
     constexpr size_t kStageMost = 160 * 1024;
     const size_t smem = size_t{kDecodeThreads} * e.floats_per_record * sizeof(float);
     const bool stage = smem <= kStageMost && (reinterpret_cast<uintptr_t>(raw) & 15u) == 0;
-    if (stage) {
+    if (stage && smem > 47 * 1024) {   // a launch may take 48 KB unasked, half a KB of it the kernel's own
         // Always the most: the limit belongs to the process, and another
         // thread may be about to decode longer records.
         const cudaError_t a = cudaFuncSetAttribute(decode_splats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -1,6 +1,7 @@
 """Launches whose shared memory goes past the limit a kernel has unasked. The
-limit belongs to the process: frames of different widths on two threads, and
-rows of harmonics from the usual 23 words to far longer, padded ones."""
+limit belongs to the process: frames of different widths on two threads, rows
+of harmonics from the usual 23 words to far longer, padded ones, and records
+from the usual 59 floats to more than a block stages."""
 from __future__ import annotations
 
 import dataclasses
@@ -71,3 +72,18 @@ def test_padded_rows_of_harmonics(rasterizer, words):
         images.append((t.colour.clone(), t.depth.clone()))
     assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
     assert float(images[0][0].abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("floats", [60, 93, 94, 95, 96, 320, 321])
+def test_padded_records(rasterizer, floats):
+    """Records decoded on the device: 128 of them are staged up to 160 KB (320 floats each)."""
+    raw = torch.from_numpy(L.synthetic_records(1000, 6)).cuda()
+    assert raw.shape[1] == 59
+    padded = torch.full((raw.shape[0], floats), 1e30, device="cuda")
+    padded[:, :59] = raw
+    encoding = L.ply_encoding(15)
+    want = rasterizer.decode_splats(raw, encoding, 15)
+    encoding.floats_per_record = floats
+    got = rasterizer.decode_splats(padded, encoding, 15)
+    for name in ("positions", "shape", "sh"):
+        assert torch.equal(getattr(got, name).view(torch.int32), getattr(want, name).view(torch.int32)), name
