@@ -31,8 +31,8 @@ struct lrt_rast {
     std::string error;
     DeviceBuffer proj, rects, touched, keys;            // per slot
     // Per pair, 8 bytes each: the pair words and the sort's other buffer; in
-    // frames made from runs (rows.cu) the runs, and every tile's slots followed
-    // by their emit indices.
+    // frames made from runs (rows.cu) the runs, and every tile's slots (4 bytes)
+    // followed, in training frames, by their emit indices.
     DeviceBuffer pairs, pairsAlt;
     DeviceBuffer ranges;                                 // per tile
     DeviceBuffer tileOrder;                              // per tile: the blend's launch order
@@ -54,9 +54,10 @@ struct lrt_rast {
     // counts copied to the host; ev[7..9]: the training backward's times.
     cudaEvent_t ev[10] = {};
     uint32_t splatCap = 0, pairCap = 0, tileCap = 0;
-    // The last single frame whose counts were read: its pairs, its splats and
-    // its runs of tiles (0 where they were not counted).
-    uint32_t seenPairs = 0, seenSlots = 0, seenRuns = 0;
+    // The last single frame whose counts were read: its pairs and its splats;
+    // and the runs of tiles and pairs of the last one of as many splats that
+    // counted its runs (0: none did).
+    uint32_t seenPairs = 0, seenSlots = 0, seenRuns = 0, seenRunPairs = 0;
     lrt_debug_view debug{};
     // Training: what the backward pass needs from its forward.
     DeviceBuffer pairValues, pairValuesAlt, pairOffsets, pixState, pixLast, partials;
@@ -174,9 +175,12 @@ inline uint32_t grow(uint32_t have, uint32_t need) {
 // A single frame's published counters (launch_publish_counters), kept for the
 // next frame's choice of form.
 inline void note_counts(lrt_rast* r, const uint32_t* counts, uint32_t slots) {
+    if (counts[4] != 0 || slots != r->seenSlots) {
+        r->seenRuns = counts[4];
+        r->seenRunPairs = counts[1];
+    }
     r->seenPairs = counts[1];
     r->seenSlots = slots;
-    r->seenRuns = counts[4];
 }
 
 inline cudaError_t ensure(DeviceBuffer& b, size_t bytes) {

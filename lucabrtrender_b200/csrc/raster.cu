@@ -167,17 +167,28 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     // A splat has at most a run a tile row where each of its rows is one run,
     // and one a tile of its rectangle where one is not (long thin splats seen
     // at a slant: up to eight times the pairs in a frame of those). Frames
-    // with more runs than pairs take words. A frame that waits may learn its
-    // runs by not holding them, and is then drawn again; one that does not
-    // wait takes words, and counts its runs, until they are known.
+    // with more than a run for every two pairs take words. Pairs ordered, in
+    // ms as runs / words, by runs a pair (200k splats, 4K, 12 to 16M pairs):
+    // 0.11 0.246 / 0.661, 0.34 0.267 / 0.405, 0.47 0.379 / 0.491, 0.51 0.381 /
+    // 0.456, 0.61 0.423 / 0.446 with 0.026 more in the projection, which
+    // counts the runs, 0.70 0.447 / 0.378; at 5M pairs 0.62 0.205 / 0.165.
+    // What is known is the count of the last frame that made one, at about
+    // this many pairs. A frame that waits may learn its runs by not holding
+    // them, and is then drawn again; one that does not wait takes words, and
+    // counts its runs, where they are not known.
     constexpr uint32_t kRunsMinPairs = 1u << 21, kRunsMinPerSplat = 6;
     const bool rowsAllowed = tilesX <= lrt::kMaxBands && tilesY <= lrt::kMaxBands;
     bool countRuns = false, byRows = false;
-    auto choose_form = [&](uint32_t pairCount, uint32_t runCount, bool waits) {
-        countRuns = rowsAllowed && pairCount >= kRunsMinPairs && pairCount / kRunsMinPerSplat >= slots;
-        byRows = countRuns && (runCount != 0 ? runCount <= pairCount : waits);
+    auto choose_form = [&](uint32_t pairCount, bool waits) {
+        const bool pays = rowsAllowed && pairCount >= kRunsMinPairs && pairCount / kRunsMinPerSplat >= slots;
+        const uint32_t quarter = pairCount / 4;
+        const bool known = r->seenRuns != 0 && r->seenRunPairs >= pairCount - quarter &&
+                           r->seenRunPairs - std::min(r->seenRunPairs, pairCount) <= quarter;
+        const bool few = known && r->seenRuns <= r->seenRunPairs / 2;
+        countRuns = pays && (!known || few);
+        byRows = pays && (known ? few : waits);
     };
-    if (r->seenSlots == slots) choose_form(r->seenPairs, r->seenRuns, !deferred);
+    if (r->seenSlots == slots) choose_form(r->seenPairs, !deferred);
 
     // Buffers (TileRasterizer.cpp:105-177).
     if (slots > r->splatCap) {
@@ -261,7 +272,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
     auto mark = [&](int k) { return s->time_stages ? cudaEventRecord(r->ev[k], stream) : cudaSuccess; };
     // Three attempts at most: one whose pairs do not fit; one with room for
     // them, as runs not counted before; and, should those be more than the
-    // pairs, one as words, with room for every pair.
+    // pairs' buffer holds, one as words, with room for every pair.
     constexpr int kAttempts = 3;
     for (int attempt = 0; attempt < kAttempts; ++attempt) {
         RowFrame rows{};
@@ -274,7 +285,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         // Both forms use the same buffers, so that a handle that draws both
         // holds them once.
         LRT_CUDA(r, ensure(r->pairs, size_t{r->pairCap} * 8), "pairs");
-        LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * 8), "pairs");
+        LRT_CUDA(r, ensure(r->pairsAlt, size_t{r->pairCap} * (byRows && !train ? 4 : 8)), "pairs");
         if (train) {
             LRT_CUDA(r, ensure(r->pairValues, size_t{r->pairCap} * 4), "pair values");
             if (!lowIsEmit && !byRows) LRT_CUDA(r, ensure(r->pairValuesAlt, size_t{r->pairCap} * 4), "pair values");
@@ -500,7 +511,7 @@ int render_frame(lrt_rast* r, const lrt_projection* pr, const std::vector<CloudD
         if ((pairs <= r->pairCap && (statusBits & lrt::kErrRuns) == 0) || attempt + 1 == kAttempts) break;
         // Draw again with room for every pair.
         r->pairCap = grow(r->pairCap, pairs);
-        choose_form(pairs, r->seenRuns, true);
+        choose_form(pairs, true);
     }
     // Rows the frame's large splats asked for beyond the row table: the next
     // frame's table holds them (this one planned those rows again).

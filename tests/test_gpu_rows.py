@@ -306,3 +306,26 @@ def test_other_frames(kind):
             assert r.debug_view().from_runs
     finally:
         r.close()
+
+
+def test_frames_of_more_than_a_run_for_two_pairs():
+    """Upright needles, nearly a run a pair: a fresh handle's first frame meets
+    their runs as it is drawn again, and the frames after it take words."""
+    n, rng = 120000, np.random.default_rng(8)
+    raw = np.zeros((n, 14), np.float32)
+    raw[:, 0:3] = 0.7 * rng.standard_normal((n, 3))
+    raw[:, 4:7] = -6.5
+    raw[:, 4] = -2.0 + 0.3 * rng.standard_normal(n)
+    half = 0.5 * (np.pi / 2 + 0.03 * rng.standard_normal(n))
+    raw[:, 7], raw[:, 10] = np.cos(half), np.sin(half)
+    raw[:, 11:14] = rng.standard_normal((n, 3))
+    sc = H.Scene("upright", [(L.pack_splats(raw, 0, 0), np.eye(4), None)], H.camera((0.2, 0.3, 4.0), focal=24.0),
+                 H.settings(1500, 1100))
+    ref = sc.oracle_render()
+    assert ref["pairs"] >= MIN_PAIRS and ref["pairs"] >= MIN_PER_SPLAT * ref["slots"], ref["pairs"]
+    r = L.TileRasterizer.create(0)
+    try:
+        for from_runs in (True, False, False):
+            assert check_parity(r, sc, ref)[2]["from_runs"] == from_runs
+    finally:
+        r.close()
